@@ -549,8 +549,8 @@ typedef struct lmm_ls_rule {
  * regressions not run), d_status (bits of lmm_ls_regress, plus 8: a
  * half-width search stopped after 512 count evaluations, where the
  * reference's search does not end, e.g. more than the upper target of net
- * values exactly zero; 16: a search needed more than its device passes) and
- * d_price = mean_p y_p / N_0(p).  Everything stays on the device: no host
+ * values exactly zero; 16: a search needed more than its device passes; 32:
+ * a bounded wait between the launch's CTAs ran out) and d_price = mean_p y_p / N_0(p).  Everything stays on the device: no host
  * synchronisation inside, so the call can be captured in a graph.
  * Workspace: lmm_ls_nested_workspace_bytes(). */
 size_t lmm_ls_nested_workspace_bytes(int paths, int n_exercise);

@@ -34,18 +34,6 @@ int reduce_launch(const float* d_in, const float* d_div, size_t n,
                   double scale, double* d_partials, double* d_out,
                   cudaStream_t stream);
 
-// Shuffle-down of a double whose two halves move in program order
-// (volatile), so a sequence of these is never interleaved by the scheduler.
-__device__ __forceinline__ double shfl_down_d_ordered(double x, int o) {
-  unsigned lo, hi;
-  asm volatile("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
-  asm volatile("shfl.sync.down.b32 %0, %0, %1, 0x1f, 0xffffffff;" : "+r"(lo) : "r"(o));
-  asm volatile("shfl.sync.down.b32 %0, %0, %1, 0x1f, 0xffffffff;" : "+r"(hi) : "r"(o));
-  double y;
-  asm volatile("mov.b64 %0, {%1, %2};" : "=d"(y) : "r"(lo), "r"(hi));
-  return y;
-}
-
 __device__ __forceinline__ double warp_sum_d(double x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
@@ -120,7 +108,7 @@ __device__ __forceinline__ float apply_decision(
 // handle the same 32 paths, so no thread holds more than 78 sums.  Sums
 // within a warp (a few paths per thread, then a fixed shuffle tree over
 // its 32 threads) are FP32; everything above them is FP64: a fixed-order
-// sum over warps, a partial per CTA in part[q][cta] and the sum over CTAs.  The CTA that finishes last (ticket on
+// sum over warps, a partial per CTA in part[cta][q] and the sum over CTAs.  The CTA that finishes last (ticket on
 // counter[e]) sums the partials in a fixed order and solves the normal
 // equations with a one-warp FP64 Cholesky, so the date needs one launch and
 // the result is independent of which CTA came last.
@@ -173,10 +161,14 @@ __device__ __forceinline__ void accumulate_rows(const float* phi, float* acc) {
 // The back substitution runs by columns of L^T from a shared-memory copy of
 // L (Ls, kMaxBasis^2 doubles of scratch).  Returns status bits (1: zero
 // diagonal, 2: not positive definite after jitter, 4: jitter added); beta
-// is zero on failure.
-__device__ int warp_cholesky_solve(const double* Gs, int K, double* beta_out, double* Ls) {
+// is zero on failure.  KC > 0: K is known at compile time (a fixed number of
+// columns without a branch each).
+template <int KC = 0>
+__device__ int warp_cholesky_solve(const double* Gs, int K_in, double* beta_out, double* Ls) {
+  constexpr int kMaxBasis = KC > 0 ? KC : lmm::kMaxBasis;  // columns
+  const int K = KC > 0 ? KC : K_in;
   const int lane = threadIdx.x & 31;
-  if (lane < kMaxBasis) beta_out[lane] = 0.0;
+  if (lane < lmm::kMaxBasis) beta_out[lane] = 0.0;
   double maxd = 0.0;
   for (int i = 0; i < K; ++i) maxd = fmax(maxd, fabs(Gs[i * kLsMaxSlots + i]));
   if (!(maxd > 0.0)) return 1;
@@ -185,6 +177,7 @@ __device__ int warp_cholesky_solve(const double* Gs, int K, double* beta_out, do
   double a[kMaxBasis];
   double rinv = 0.0;  // this lane's 1 / L_ii
   bool ok = false;
+#pragma unroll 1
   for (int attempt = 0; attempt < 6 && !ok; ++attempt) {
 #pragma unroll
     for (int k = 0; k < kMaxBasis; ++k)
@@ -196,9 +189,9 @@ __device__ int warp_cholesky_solve(const double* Gs, int K, double* beta_out, do
     for (int j = 0; j < kMaxBasis; ++j) {
       if (j < K) {
         const double djj = __shfl_sync(0xffffffffu, a[j], j);
-        if (!(djj > 1e-300)) {
+        if (!(djj > 1e-300)) {  // with KC the remaining columns run on, unused
           ok = false;
-          break;
+          if (KC == 0) break;
         }
         const double rj = rsqrt(djj);
         if (lane == j) {
@@ -251,8 +244,70 @@ __device__ int warp_cholesky_solve(const double* Gs, int K, double* beta_out, do
       if (lane < i) z -= lcol[i] * bi;
     }
   }
-  if (lane < kMaxBasis) beta_out[lane] = (lane < K) ? bet : 0.0;
+  if (lane < lmm::kMaxBasis) beta_out[lane] = (lane < K) ? bet : 0.0;
   return status;
+}
+
+// acc[0 .. N) summed over the warp's lanes by exchanging halves of the
+// accumulators (67 shuffles for 66 sums instead of five each): the lane is
+// left with the sums q = first .. first + count - 1 in acc[0 .. count).  Every
+// sum is the binary tree over lanes l and l + 16, then + 8, ..., + 1.
+template <int N, class V>
+__device__ __forceinline__ void warp_sums_range(int o, int& first, int& count) {
+  constexpr int H = (N + 1) / 2;
+  if (threadIdx.x & o) {
+    first += H;
+    count = max(count - H, 0);
+  } else {
+    count = min(count, H);
+  }
+}
+template <int N, class V>
+__device__ __forceinline__ void warp_sums_step(V* acc, int o, int& first, int& count) {
+  constexpr int H = (N + 1) / 2;
+  const bool up = (threadIdx.x & o) != 0;
+#pragma unroll
+  for (int i = 0; i < H; ++i) {
+    const V hi = H + i < N ? acc[H + i] : V(0);
+    const V send = up ? acc[i] : hi, keep = up ? hi : acc[i];
+    acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+  }
+  warp_sums_range<N, V>(o, first, count);
+}
+template <int N>
+constexpr int warp_sums_left() {  // five halvings
+  return ((((((((((N + 1) / 2) + 1) / 2) + 1) / 2) + 1) / 2) + 1) / 2);
+}
+template <int N>
+__device__ __forceinline__ void warp_sums(float* acc, int& first, int& count) {
+  first = 0;
+  count = N;
+  constexpr int N1 = (N + 1) / 2, N2 = (N1 + 1) / 2, N3 = (N2 + 1) / 2, N4 = (N3 + 1) / 2;
+  warp_sums_step<N>(acc, 16, first, count);
+  warp_sums_step<N1>(acc, 8, first, count);
+  warp_sums_step<N2>(acc, 4, first, count);
+  warp_sums_step<N3>(acc, 2, first, count);
+  warp_sums_step<N4>(acc, 1, first, count);
+}
+// the same with the sums in FP64 (the lanes' values still FP32)
+template <int N>
+__device__ __forceinline__ void warp_sums_d(const float* acc, double (&d)[(N + 1) / 2],
+                                            int& first, int& count) {
+  constexpr int N1 = (N + 1) / 2, N2 = (N1 + 1) / 2, N3 = (N2 + 1) / 2, N4 = (N3 + 1) / 2;
+  const bool up = (threadIdx.x & 16) != 0;
+#pragma unroll
+  for (int i = 0; i < N1; ++i) {
+    const float hi = N1 + i < N ? acc[N1 + i] : 0.0f;
+    const float send = up ? acc[i] : hi, keep = up ? hi : acc[i];
+    d[i] = (double)keep + (double)__shfl_xor_sync(0xffffffffu, send, 16);
+  }
+  first = 0;
+  count = N;
+  warp_sums_range<N, double>(16, first, count);
+  warp_sums_step<N1>(d, 8, first, count);
+  warp_sums_step<N2>(d, 4, first, count);
+  warp_sums_step<N3>(d, 2, first, count);
+  warp_sums_step<N4>(d, 1, first, count);
 }
 
 // Staged loop of the date kernel: the inputs of a path, one shared-memory
@@ -272,24 +327,12 @@ constexpr size_t ls_stage_bytes() {
          (kLsInputs * sizeof(float) + (MASKED ? sizeof(double) : 0));
 }
 
-__device__ __forceinline__ void cp_async4(float* dst_smem, const float* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(float* dst_smem, const float* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(double* dst_smem, const double* src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+// With rows split over a warp pair only the first warp writes a path's running
+// value, in the place both read it from: the pair meets in every iteration,
+// so that the second warp's copy of the stage is in before the write.
+template <int NSPLIT>
+__device__ __forceinline__ void pair_sync(int warp) {
+  if (NSPLIT == 2) asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp >> 1)) : "memory");
 }
 
 template <int KR, int NSPLIT, int KIND, bool MASKED>
@@ -436,6 +479,7 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
       issue(it + kLsStages - 1, qw + (kLsStages - 1) * stride);
       cp_async_wait<kLsStages - 1>();
       __syncwarp();
+      pair_sync<NSPLIT>(warp);
       const int p = qw + lane;
       const bool member =
           !MASKED || (p < paths && fabs(mstage[(it & (kLsStages - 1)) * kLsThreads + tid]) <= cut);
@@ -468,29 +512,23 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
     }
     cp_async_wait<0>();
   }
-  // warp sums (a fixed shuffle tree), then FP64 over warps in a fixed
-  // order.  All-path launches sum within the warp in FP32 (each thread
-  // holds several paths' FP32 sums already).  Masked launches (nested
-  // regressions on a subset, about one path per thread) sum in FP64, one
-  // accumulator at a time: their Grams are close to singular, and the FP32
-  // tree would be their largest rounding error.
+  // warp sums (a fixed tree), then FP64 over warps in a fixed order.
+  // All-path launches sum within the warp in FP32 (each thread holds several
+  // paths' FP32 sums already).  Masked launches (nested regressions on a
+  // subset, about one path per thread) sum in FP64: their Grams are close to
+  // singular, and the FP32 tree would be their largest rounding error.
+  int first, count;
   if (MASKED) {
+    double d[(NA + 1) / 2];
+    warp_sums_d<NA>(acc, d, first, count);
 #pragma unroll
-    for (int q = 0; q < NA; ++q) {
-      double t;
-      asm volatile("cvt.f64.f32 %0, %1;" : "=d"(t) : "f"(acc[q]));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += shfl_down_d_ordered(t, o);
-      if (lane == 0) red_s[warp][q] = t;
-    }
+    for (int i = 0; i < warp_sums_left<NA>(); ++i)
+      if (i < count) red_s[warp][first + i] = d[i];
   } else {
+    warp_sums<NA>(acc, first, count);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int q = 0; q < NA; ++q) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < NA; ++q) red_s[warp][q] = (double)acc[q];
+    for (int i = 0; i < warp_sums_left<NA>(); ++i)
+      if (i < count) red_s[warp][first + i] = (double)acc[i];
   }
   __syncthreads();
   const int nb = gridDim.x;
@@ -499,7 +537,7 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
     const int qq = h ? q - RowSplit<KR, 0, RS>::n : q;
     double s = 0.0;
     for (int w = h; w < NW; w += NSPLIT) s += red_s[w][qq];
-    part[(size_t)q * nb + blockIdx.x] = s;
+    part[(size_t)blockIdx.x * NPAIRS + q] = s;
   }
   // last CTA: sum the partials and solve.  The CTA barrier orders every
   // thread's partial writes before thread 0's device-scope fence and ticket
@@ -513,25 +551,23 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
   __syncthreads();
   if (!last_s) return;
   __threadfence();
-  // tpq threads per pair, each summing a strided share of the CTA partials
-  // with its loads unrolled (one pass of L2 latency, not one per partial),
-  // then the shares of a pair in a fixed order
+  // thread (sub, q) adds every tpq-th CTA's partial of pair q, its loads
+  // coalesced and unrolled (one pass of L2 latency, not one per partial), then
+  // the shares of a pair follow in a fixed order
   {
-    const int tpq = kLsThreads / NPAIRS;
-    double* share = share_s;
-    const int q = tid / tpq, sub = tid - q * tpq;
+    constexpr int tpq = kLsThreads / NPAIRS;
+    const int sub = tid / NPAIRS, q = tid - sub * NPAIRS;
     double v = 0.0;
-    if (q < NPAIRS) {
-      const double* src = part + (size_t)q * nb;
-#pragma unroll 8
-      for (int b = sub; b < nb; b += tpq) v += __ldcg(src + b);
+    if (sub < tpq) {
+      const double* src = part + q;
+#pragma unroll 11
+      for (int b = sub; b < nb; b += tpq) v += __ldcg(src + (size_t)b * NPAIRS);
     }
-    __syncthreads();
-    share[tid] = v;
+    share_s[tid] = v;
     __syncthreads();
     if (tid < NPAIRS) {
       double t = 0.0;
-      for (int k = 0; k < tpq; ++k) t += share[tid * tpq + k];
+      for (int k = 0; k < tpq; ++k) t += share_s[k * NPAIRS + tid];
       sums_s[tid] = t;
     }
   }

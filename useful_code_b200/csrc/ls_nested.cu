@@ -16,20 +16,18 @@
 // Per date e the loop is a fixed sequence of launches with no host
 // synchronisation: the decision of date e + 1 is applied to the running
 // values; the first regression runs over all paths (ls_date_kernel); then
-// for each further depth d: a pass forms the net values of regression d - 1
-// on its paths (non-members hold +inf) with their FP64 moments; a few
-// selection passes count |net| against up to 256 thresholds each (one
-// histogram per pass) and advance the half-width search, which the last CTA
-// of each pass runs exactly as the reference's sequential search, reading
-// counts from the histogram; the moments of the selected paths follow,
-// then the regression over them (ls_date_kernel with a mask).  When a date
-// stops nesting (one-sign net values, too few paths, or a search that did
-// not finish), a flag makes its remaining launches return at once.
+// for each further depth d one cooperative launch (nested_select_kernel)
+// takes the net values of regression d - 1 on its paths, searches the
+// half-width of the band of paths to regress again, and forms the moments
+// of the selected paths; then the regression over them (ls_date_kernel with
+// a mask).  When a date stops nesting (one-sign net values, too few paths,
+// or a search that did not finish), a flag makes its remaining launches
+// return at once.
 //
 // The reference's search evaluates one count per step on the whole path
 // set.  Here each pass evaluates every count the search can ask for next:
-// the whole geometric chain of its grow or shrink loop, or the next eight
-// levels of its bisection tree, computed with the same floating-point
+// a stretch of the geometric chain of its grow or shrink loop, or the next
+// eight levels of its bisection tree, computed with the same floating-point
 // operations, so the search reads exact counts and takes the same steps.
 #include "lmm_common.cuh"
 #include "lmm_device.cuh"
@@ -51,161 +49,42 @@ using namespace lmm;
 namespace {
 
 constexpr int kSelBatch = 256;      // thresholds per selection pass
-constexpr int kSelPasses = 6;       // selection passes launched per depth
+constexpr int kSelChain = 48;       // of them in a chain pass
+constexpr int kSelPasses = 16;      // selection passes of a search at most
 constexpr int kSelMaxCounts = 512;  // count evaluations per search
 constexpr int kSelCapped = 8;       // status: a search stopped at kSelMaxCounts
 constexpr int kSelIncomplete = 16;  // status: a search needed more passes
-constexpr int kNestThreads = 256;
+constexpr int kSelWait = 32;        // status: a wait of the grid ran out
+constexpr int kNestThreads = 256;   // decision kernel
+constexpr int kSelThreads = 512;    // selection kernel, one CTA per SM
 
+// State of the search for one (date, depth), the same in every CTA's shared
+// memory.  A pass counts |net| against the ascending thresholds thr[0 .. nb);
+// chain passes hold a geometric chain, tree passes the next eight levels of
+// the bisection of [lo, hi] in symmetric order.
 enum {
   kPhDone = 0,
-  kPhBranch,      // n within the targets: the reference keeps every path (cut 1e4)
-  kPhInit,        // count at g = sds * sd
-  kPhGrow,        // g /= multiplier while count < lower target
-  kPhShrinkInit,  // count at lo = g * multiplier
-  kPhShrink,      // lo *= multiplier while count > upper target
-  kPhBisectInit,  // count at g = (lo + hi) / 2
-  kPhBisect       // halve [lo, hi] while the count is outside the targets
+  kPhBranch,  // n within the targets: the reference keeps every path (cut 1e4)
+  kPhInit,    // g at thr[nb - 1] and the shrinking chain g m, g m^2, ... below it
+  kPhGrow,    // g / m, g / m^2, ... (the count at g was below the lower target)
+  kPhShrink,  // lo m, lo m^2, ... (the count at lo is above the upper target)
+  kPhTree     // halvings of [lo, hi]
 };
-
-// Search state of one (date, depth), kept in the workspace between passes.
 struct SelState {
   int phase, lo_t, hi_t, evals, c, after, nb, status;
   double g, lo, hi, mult, cut;
-  double thr[kSelBatch];  // thresholds of the pending pass, ascending
-  int cnt[kSelBatch];     // paths with |net| <= thr[i], after the pass
 };
 
-__device__ bool sel_lookup(const SelState& S, double g, int* c) {
-  int a = 0, b = S.nb - 1;
-  while (a <= b) {
-    const int m = (a + b) >> 1;
-    const double t = S.thr[m];
-    if (t == g) {
-      *c = S.cnt[m];
-      return true;
-    }
-    if (t < g)
-      a = m + 1;
-    else
-      b = m - 1;
-  }
-  return false;
-}
-
-// Runs the search from its saved phase until it ends (true) or needs a
-// count the last pass did not evaluate (false; the state then says which).
-// Same steps and stopping rules as frac_select of the CPU restatement.
-__device__ bool sel_run(SelState& S) {
-  int c;
-  for (;;) {
-    switch (S.phase) {
-      case kPhBranch:
-        if (!sel_lookup(S, 1e4, &c)) return false;
-        S.cut = 1e4;
-        S.after = c;
-        S.phase = kPhDone;
-        return true;
-      case kPhInit:
-        if (!sel_lookup(S, S.g, &c)) return false;
-        ++S.evals;
-        S.c = c;
-        S.phase = kPhGrow;
-        break;
-      case kPhGrow:
-        if (S.c < S.lo_t) {
-          if (S.evals >= kSelMaxCounts) {
-            S.status |= kSelCapped;
-          } else {
-            const double g2 = S.g / S.mult;
-            if (!sel_lookup(S, g2, &c)) return false;
-            S.g = g2;
-            S.c = c;
-            ++S.evals;
-            break;
-          }
-        }
-        if (S.c < S.hi_t) {
-          S.cut = S.g;
-          S.after = S.c;
-          S.phase = kPhDone;
-          return true;
-        }
-        S.lo = S.g * S.mult;
-        S.phase = kPhShrinkInit;
-        break;
-      case kPhShrinkInit:
-        if (!sel_lookup(S, S.lo, &c)) return false;
-        ++S.evals;
-        S.c = c;
-        S.phase = kPhShrink;
-        break;
-      case kPhShrink:
-        if (S.c > S.hi_t) {
-          if (S.evals >= kSelMaxCounts) {
-            S.status |= kSelCapped;
-          } else {
-            const double l2 = S.lo * S.mult;
-            if (!sel_lookup(S, l2, &c)) return false;
-            S.lo = l2;
-            S.c = c;
-            ++S.evals;
-            break;
-          }
-        }
-        if (S.c > S.lo_t) {
-          S.cut = S.lo;
-          S.after = S.c;
-          S.phase = kPhDone;
-          return true;
-        }
-        S.hi = S.g;
-        S.g = 0.5 * (S.lo + S.hi);
-        S.phase = kPhBisectInit;
-        break;
-      case kPhBisectInit:
-        if (!sel_lookup(S, S.g, &c)) return false;
-        ++S.evals;
-        S.c = c;
-        S.phase = kPhBisect;
-        break;
-      case kPhBisect:
-        if ((S.c < S.lo_t || S.c > S.hi_t) && (S.hi - S.lo) > 1e-6) {
-          if (S.evals >= kSelMaxCounts) {
-            S.status |= kSelCapped;
-          } else {
-            if (S.c < S.lo_t)
-              S.lo = S.g;
-            else
-              S.hi = S.g;
-            S.g = 0.5 * (S.lo + S.hi);
-            S.phase = kPhBisectInit;
-            break;
-          }
-        }
-        S.cut = S.g;
-        S.after = S.c;
-        S.phase = kPhDone;
-        return true;
-      default:
-        return true;
-    }
-  }
-}
-
-// Thresholds the search can ask for next from its saved phase, written
-// unsorted to out (thread 0 for the chains; the bisection tree in
-// parallel, node i by the halvings on its path from the root).  Returns
-// the count.
-__device__ int sel_batch(const SelState& S, double* out) {
+// Thresholds of the phase's next pass, with the floating-point operations of
+// the sequential search.  All threads of the CTA; ends with a barrier.
+__device__ void sel_thresholds(SelState& S, double* thr) {
   const int tid = threadIdx.x;
-  int n = 0;
-  if (S.phase == kPhBisectInit) {
-    // node i (heap order): from [lo, hi], left child = [lo, mid] (the count
-    // was above the upper target), right child = [mid, hi]
-    for (int i = tid; i < kSelBatch - 1; i += blockDim.x) {
-      const int h = i + 1;
-      int lead = 31 - __clz(h);
+  if (S.phase == kPhTree) {
+    // node h (heap order, 1-based) of [lo, hi]: left child = [lo, mid] (the
+    // count was above the upper target), right child = [mid, hi]; its rank
+    // in symmetric order from its level and place
+    for (int h = tid + 1; h < kSelBatch; h += blockDim.x) {
+      const int lead = 31 - __clz(h);
       double lo = S.lo, hi = S.hi;
       for (int b = lead - 1; b >= 0; --b) {
         const double mid = 0.5 * (lo + hi);
@@ -214,102 +93,208 @@ __device__ int sel_batch(const SelState& S, double* out) {
         else
           hi = mid;
       }
-      out[i] = 0.5 * (lo + hi);
+      thr[((2 * (h - (1 << lead)) + 1) << (7 - lead)) - 1] = 0.5 * (lo + hi);
     }
-    return kSelBatch - 1;
-  }
-  if (tid == 0) {
-    switch (S.phase) {
-      case kPhBranch:
-        out[n++] = 1e4;
-        break;
-      case kPhInit: {
-        out[n++] = S.g;
-        double g = S.g;
-        for (int i = 0; i < 63; ++i) {
-          g = g / S.mult;
-          out[n++] = g;
-        }
-        double l = S.g * S.mult;
-        out[n++] = l;
-        while (n < kSelBatch) {
-          l = l * S.mult;
-          out[n++] = l;
-        }
-        break;
-      }
-      case kPhGrow: {
-        double g = S.g;
-        while (n < kSelBatch) {
-          g = g / S.mult;
-          out[n++] = g;
-        }
-        break;
-      }
-      case kPhShrinkInit: {
-        double l = S.lo;
-        out[n++] = l;
-        while (n < kSelBatch) {
-          l = l * S.mult;
-          out[n++] = l;
-        }
-        break;
-      }
-      case kPhShrink: {
-        double l = S.lo;
-        while (n < kSelBatch) {
-          l = l * S.mult;
-          out[n++] = l;
-        }
-        break;
-      }
-      default:
-        break;
+    if (tid == 0) S.nb = kSelBatch - 1;
+  } else if (tid == 0) {
+    int n = kSelBatch;
+    if (S.phase == kPhBranch) {
+      thr[0] = 1e4;
+      n = 1;
+    } else if (S.phase == kPhGrow) {
+      double g = S.g;
+      n = kSelChain;
+      for (int i = 0; i < n; ++i) thr[i] = g = g / S.mult;
+    } else {
+      n = kSelChain;
+      double l = S.phase == kPhInit ? S.g : S.lo * S.mult;
+      for (int i = n - 1; i >= 0; --i, l *= S.mult) thr[i] = l;
     }
+    S.nb = n;
   }
-  return n;
+  __syncthreads();
 }
 
-// Sorts the pending thresholds into S.thr (rank by counting; ties keep
-// their order) after sel_batch wrote them to tmp.  All threads of the block.
-__device__ void sel_prepare(SelState& S, double* tmp, int* n_s) {
-  const int n = sel_batch(S, tmp);
-  if (threadIdx.x == 0) *n_s = n;
-  __syncthreads();
-  const int nb = *n_s;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    const double v = tmp[i];
-    int r = 0;
-    for (int j = 0; j < nb; ++j) r += (tmp[j] < v) || (tmp[j] == v && j < i);
-    S.thr[r] = v;
+// Advances the search (thread 0 of every CTA alike) from the counts cnt[i] of
+// paths with |net| <= thr[i]; the same steps and stopping rules as
+// frac_select of the CPU restatement.  Leaves kPhDone, or the phase of the
+// pass whose counts it needs next.
+__device__ __forceinline__ void sel_step(SelState& S, const double* thr, const int* cnt) {
+  auto done = [&](double cut, int after) {
+    S.cut = cut;
+    S.after = after;
+    S.phase = kPhDone;
+  };
+  auto capped = [&]() {
+    if (S.evals < kSelMaxCounts) return false;
+    S.status |= kSelCapped;
+    return true;
+  };
+  auto bisect = [&]() {  // from the chain's bracket
+    S.hi = S.g;
+    S.phase = kPhTree;
+  };
+  // after a shrink step left the count S.c at S.lo
+  auto shrunk = [&]() {
+    if (S.c > S.lo_t)
+      done(S.lo, S.c);
+    else
+      bisect();
+  };
+  // walk down the chain thr[i], thr[i - 1], ... of candidates for lo
+  auto shrink = [&](int i) {
+    for (;;) {
+      if (!(S.c > S.hi_t) || capped()) return shrunk();
+      if (i < 0) {
+        S.phase = kPhShrink;  // from S.lo
+        return;
+      }
+      S.lo = thr[i];
+      S.c = cnt[i--];
+      ++S.evals;
+    }
+  };
+  const int top = S.nb - 1;
+  switch (S.phase) {
+    case kPhBranch:
+      return done(1e4, cnt[0]);
+    case kPhInit:
+      S.c = cnt[top];
+      ++S.evals;
+      if (S.c < S.lo_t) {
+        S.phase = kPhGrow;
+        return;
+      }
+      if (S.c < S.hi_t) return done(S.g, S.c);
+      S.lo = thr[top - 1];
+      S.c = cnt[top - 1];
+      ++S.evals;
+      return shrink(top - 2);
+    case kPhGrow: {
+      int i = 0;
+      while (S.c < S.lo_t && !capped()) {
+        if (i > top) return;  // more of the chain, from S.g
+        S.g = thr[i];
+        S.c = cnt[i++];
+        ++S.evals;
+      }
+      if (S.c < S.hi_t) return done(S.g, S.c);
+      // lo = g m need not be a threshold of this pass: start the chain below g
+      --S.evals;
+      S.phase = kPhInit;
+      return;
+    }
+    case kPhShrink:
+      return shrink(top);
+    default: {
+      int h = 1;  // tree node whose midpoint is asked for
+      for (;;) {
+        if (h >= kSelBatch) return;  // eight levels used: next pass from [lo, hi]
+        const int lead = 31 - __clz(h);
+        const int i = ((2 * (h - (1 << lead)) + 1) << (7 - lead)) - 1;
+        S.g = thr[i];
+        S.c = cnt[i];
+        ++S.evals;
+        if (!((S.c < S.lo_t || S.c > S.hi_t) && (S.hi - S.lo) > 1e-6) || capped())
+          return done(S.g, S.c);
+        if (S.c < S.lo_t) {
+          S.lo = S.g;
+          h = 2 * h + 1;
+        } else {
+          S.hi = S.g;
+          h = 2 * h;
+        }
+      }
+    }
   }
-  if (threadIdx.x == 0) S.nb = nb;
+}
+
+__device__ void sel_advance(SelState& shared, const double* thr, const int* cnt) {
+  SelState S = shared;  // in registers
+  sel_step(S, thr, cnt);
+  shared = S;
+}
+
+// Barrier of a cooperative grid: generation `gen` (1, 2, ... in this launch)
+// is over when the counter has reached gen * gridDim.x.  Every CTA arrives
+// once per generation.  The wait is bounded: false when it ran out (it cannot
+// while all CTAs are resident and arrive).
+__device__ bool grid_wait(unsigned int* counter, unsigned gen, int* ok_s) {
   __syncthreads();
+  if (threadIdx.x == 0) {
+    const unsigned want = gen * gridDim.x;
+    __threadfence();
+    atomicAdd(counter, 1u);
+    int ok = 0;
+    for (int i = 0; i < (1 << 22) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
+    __threadfence();
+    *ok_s = ok;
+  }
+  __syncthreads();
+  return *ok_s != 0;
 }
 
 // Ticket of the grid: true in the last CTA to arrive (after its partials
 // are visible to it).
 __device__ bool last_block(unsigned int* ticket, int* flag_s) {
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) *flag_s = (atomicAdd(ticket, 1u) == gridDim.x - 1u);
+  if (threadIdx.x == 0) {
+    __threadfence();
+    *flag_s = (atomicAdd(ticket, 1u) == gridDim.x - 1u);
+    __threadfence();
+  }
   __syncthreads();
-  if (!*flag_s) return false;
-  __threadfence();
-  return true;
+  return *flag_s != 0;
 }
 
-__device__ __forceinline__ double block_sum(double x, double* red_s) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+// Sums over the block of NV values per thread, in out_s[0 .. NV) after the
+// call (all threads): a shuffle tree per warp, then the warps in order.
+// red_s holds NV x warps.
+template <int NV>
+__device__ void block_sums(const double (&x)[NV], double* red_s, double* out_s) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  double t[NV];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+  for (int i = 0; i < NV; ++i) t[i] = x[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) t[i] += __shfl_down_sync(0xffffffffu, t[i], o);
   __syncthreads();
-  if (lane == 0) red_s[w] = x;
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) red_s[i * nw + w] = t[i];
   __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red_s[i];
-  return t;  // valid in thread 0
+  if ((int)threadIdx.x < NV) {
+    double s = 0.0;
+    for (int i = 0; i < nw; ++i) s += red_s[threadIdx.x * nw + i];
+    out_s[threadIdx.x] = s;
+  }
+  __syncthreads();
+}
+
+// The same for maxima.
+template <int NV>
+__device__ void block_maxima(const double (&x)[NV], double* red_s, double* out_s) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  double t[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) t[i] = x[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) t[i] = fmax(t[i], __shfl_down_sync(0xffffffffu, t[i], o));
+  __syncthreads();
+  if (lane == 0)
+#pragma unroll
+    for (int i = 0; i < NV; ++i) red_s[i * nw + w] = t[i];
+  __syncthreads();
+  if ((int)threadIdx.x < NV) {
+    double m = red_s[threadIdx.x * nw];
+    for (int i = 1; i < nw; ++i) m = fmax(m, red_s[threadIdx.x * nw + i]);
+    out_s[threadIdx.x] = m;
+  }
+  __syncthreads();
 }
 
 // Per-thread sums over CTAs of the NC columns of per-CTA partials (rows
@@ -336,73 +321,103 @@ __device__ void thread_partials(const double* part, int stride, int nblocks, dou
     for (int c = 0; c < NC; ++c) t[c] += __ldcg(part + (size_t)b * stride + c);
 }
 
-__device__ double block_max(double x, double* red_s) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = fmax(x, __shfl_down_sync(0xffffffffu, x, o));
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red_s[threadIdx.x >> 5] = x;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) x = fmax(x, red_s[i]);
-  return x;  // valid in thread 0
-}
-
-// Search state copied between global and shared memory by the whole block.
-__device__ void copy_state(SelState* dst, const SelState* src) {
-  static_assert(sizeof(SelState) % 4 == 0, "SelState is copied as words");
-  const unsigned* a = (const unsigned*)src;
-  unsigned* b = (unsigned*)dst;
-  for (int i = threadIdx.x; i < (int)(sizeof(SelState) / 4); i += blockDim.x) b[i] = a[i];
-}
-
 // Apply date e's frozen decision (depth chain, no shift) to the running
 // values and deflate them to date e - 1 when `deflate`
 // (updateDeflatedNextStepValuesMulti_gold then
 // updateDeflationOfContinuationValues_gold).
 __global__ void __launch_bounds__(kNestThreads)
-    nested_decide_kernel(const __grid_constant__ LSDate dd, int e, int deflate,
+    nested_decide_kernel(const __grid_constant__ LSDate dd, int kind, int e, int deflate,
                          const LsRuleView rule, const float* __restrict__ vars,
                          const float* __restrict__ cf, const float* __restrict__ ex,
                          const float* __restrict__ num, float* __restrict__ y, int paths) {
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < paths; p += gridDim.x * blockDim.x) {
-    float v[kMaxVars];
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long p0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; p0 < paths;
+       p0 += 2 * stride) {
+    const bool two = p0 + stride < paths;
+    const size_t p[2] = {(size_t)p0, (size_t)(two ? p0 + stride : p0)};
+    float v[2][kMaxVars], exv[2], t[2], ratio[2];
 #pragma unroll
-    for (int k = 0; k < kMaxVars; ++k)
-      v[k] = k < dd.nvars ? vars[((size_t)e * kMaxVars + k) * paths + p] : 0.0f;
-    const float exv = ex ? ex[(size_t)e * paths + p] : 0.0f;
-    const double est = ls_chain_estimate(rule, e, dd.nvars, dd.nbasis, dd.mono, v, exv);
-    const float t = (cf ? cf[(size_t)e * paths + p] : 0.0f) + y[p];
-    float yy = ((double)exv > est) ? exv : t;
-    if (deflate) yy = yy * (num[(size_t)(e - 1) * paths + p] / num[(size_t)e * paths + p]);
-    y[p] = yy;
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int k = 0; k < kMaxVars; ++k)
+        v[h][k] = k < dd.nvars ? vars[((size_t)e * kMaxVars + k) * paths + p[h]] : 0.0f;
+      exv[h] = ex ? ex[(size_t)e * paths + p[h]] : 0.0f;
+      t[h] = (cf ? cf[(size_t)e * paths + p[h]] : 0.0f) + y[p[h]];
+      ratio[h] = deflate ? num[(size_t)(e - 1) * paths + p[h]] / num[(size_t)e * paths + p[h]]
+                         : 1.0f;
+    }
+    double est[2];
+    ls_chain_estimate2(rule, e, kind, dd.nvars, dd.nbasis, dd.mono, v, exv, est);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h && !two) break;
+      const float yy = ((double)exv[h] > est[h]) ? exv[h] : t[h];
+      y[p[h]] = deflate ? yy * ratio[h] : yy;
+    }
   }
 }
 
 struct NestArgs {
   LSDate dd;
-  int e, d, rows, paths, min_paths, last;
+  int kind;  // ls_basis_kind of the date's table
+  int e, d, rows, paths, min_paths;
   double lower_frac, upper_frac, sds, mult;
 };
 
-// Net values est - exercise value of regression d at date e on its paths
-// (d = 0: all; else |net| <= cut of d - 1, net holding d - 1's values),
-// +inf elsewhere; the last CTA applies the one-sign shortcut (d = 0) and
-// starts the half-width search.
-__global__ void __launch_bounds__(kNestThreads, 4)
-    nested_net_kernel(const __grid_constant__ NestArgs a, const float* __restrict__ vars,
-                      const float* __restrict__ ex, const double* __restrict__ beta,
-                      const float* __restrict__ means, const float* __restrict__ sds,
-                      const double* __restrict__ cuts, const int* __restrict__ npaths,
-                      double* __restrict__ net, double* __restrict__ part,
-                      unsigned int* __restrict__ ticket, int* __restrict__ stopped,
-                      SelState* __restrict__ state) {
+// Barrier counter, ticket and histograms of one selection launch, zero when
+// it starts: a regression holds two, and each launch clears the one that the
+// next launch uses.
+struct NestSync {
+  unsigned int barrier, ticket;
+  int hist[kSelPasses][kSelBatch];
+};
+
+// From regression d to the paths of regression d + 1 of date e, one
+// cooperative launch (one CTA per SM, each thread keeps the same paths
+// throughout):
+//  * the net values est - exercise value of regression d on its paths
+//    (d = 0: all; else |net| <= cut of d - 1, net holding d - 1's values),
+//    +inf elsewhere, and their FP64 moments; the one-sign shortcut (d = 0);
+//  * the half-width search: each pass counts |net| against up to 256
+//    thresholds (a shared-memory histogram per CTA, integer atomics into the
+//    pass's global one, whose totals do not depend on the order), and every
+//    CTA advances the same search from the totals.  More than min_paths
+//    paths selected: cuts of regression d and the path count of regression
+//    d + 1; otherwise the date stops nesting;
+//  * the moments of the basis variables over the selected paths (means /
+//    sds row d + 1; GenerateLSRegressionMatrixSelectivelyNormalisingVariables_
+//    gold, gold/LS_regression.h:524-600), joined by the last CTA.
+// The passes stream 8-32 MB that sit in L2 and are bound by latency: with one
+// launch each for the net values, six selection passes and the moments a
+// depth paid eight launch gaps, as many serial tails (a ticket, one thread
+// sorting and looking up thresholds, state through global memory) and the
+// idle passes.  Here a pass ends with a grid barrier of about 2 us, two to
+// three passes per search.  The regression (80 dates, depth 4), together with
+// the known basis tables in the net values and decisions and the shorter
+// tails of ls_date_kernel: 33.8 -> 14.3 ms at 2^18 paths, 46.3 -> 23.6 ms at
+// 2^20, 11.9 -> 5.2 ms for 40 dates at 30,001.
+__global__ void __launch_bounds__(kSelThreads, 1)
+    nested_select_kernel(const __grid_constant__ NestArgs a, const float* __restrict__ vars,
+                         const float* __restrict__ ex, const double* __restrict__ beta,
+                         float* means, float* sds, double* cuts, int* npaths, double* net,
+                         double* part, NestSync* sync, NestSync* next, int* stopped,
+                         int* status) {
+  constexpr int NW = kSelThreads / 32;
   __shared__ double beta_s[kMaxBasis];
   __shared__ float mom_s[2][kMaxVars];
-  __shared__ double red_s[kNestThreads / 32];
+  __shared__ double red_s[2 * kMaxVars * NW];
+  __shared__ double out_s[2 * kMaxVars];
+  __shared__ int before_s[NW];
+  __shared__ double thr_s[kSelBatch];
+  __shared__ int hist_s[kSelBatch];
   __shared__ SelState S;
-  __shared__ double tmp_s[kSelBatch];
-  __shared__ int flag_s, n_s;
+  __shared__ int flag_s;
   const int e = a.e, d = a.d, paths = a.paths, tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+  if (blockIdx.x == 0)
+    for (int i = tid; i < (int)(sizeof(NestSync) / 4); i += kSelThreads)
+      reinterpret_cast<unsigned*>(next)[i] = 0u;
+  // uniform over the grid: this launch sets the flag after a barrier only
   if (stopped[e]) return;
   const size_t row = (size_t)e * a.rows + d;
   if (tid < kMaxBasis) beta_s[tid] = beta[row * kMaxBasis + tid];
@@ -411,217 +426,169 @@ __global__ void __launch_bounds__(kNestThreads, 4)
     mom_s[1][tid] = means ? sds[row * kMaxVars + tid] : 1.0f;
   }
   __syncthreads();
-  const double cut = d > 0 ? cuts[(row - 1) * 2 + 1] : 0.0;
+  const double cut0 = d > 0 ? cuts[(row - 1) * 2 + 1] : 0.0;
+  const long long p_begin = (long long)blockIdx.x * kSelThreads + tid;
+  const long long stride = (long long)gridDim.x * kSelThreads;
+  // the net values of two paths at a time
+  const LsRuleView one{1, beta_s, means ? mom_s[0] : nullptr, mom_s[1], nullptr, nullptr};
   double s1 = 0.0, s2 = 0.0, mx = -INFINITY, mn = INFINITY;
-  for (int p = blockIdx.x * blockDim.x + tid; p < paths; p += gridDim.x * blockDim.x) {
-    const bool member = d == 0 || fabs(net[p]) <= cut;
-    double nv = INFINITY;
-    if (member) {
-      float v[kMaxVars];
+  for (long long p0 = p_begin; p0 < paths; p0 += 2 * stride) {
+    const bool two = p0 + stride < paths;
+    const size_t p[2] = {(size_t)p0, (size_t)(two ? p0 + stride : p0)};
+    float v[2][kMaxVars], exv[2];
+    bool member[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      member[h] = d == 0 || fabs(net[p[h]]) <= cut0;
 #pragma unroll
       for (int k = 0; k < kMaxVars; ++k)
-        v[k] = k < a.dd.nvars ? vars[((size_t)e * kMaxVars + k) * paths + p] : 0.0f;
-      const float exv = ex ? ex[(size_t)e * paths + p] : 0.0f;
-      nv = ls_row_estimate(beta_s, means ? mom_s[0] : nullptr, mom_s[1], a.dd.nvars,
-                           a.dd.nbasis, a.dd.mono, v) -
-           (double)exv;
-      s1 += nv;
-      s2 += nv * nv;
-      mx = fmax(mx, nv);
-      mn = fmin(mn, nv);
+        v[h][k] = k < a.dd.nvars ? vars[((size_t)e * kMaxVars + k) * paths + p[h]] : 0.0f;
+      exv[h] = ex ? ex[(size_t)e * paths + p[h]] : 0.0f;
     }
-    net[p] = nv;
-  }
-  const double t1 = block_sum(s1, red_s), t2 = block_sum(s2, red_s);
-  // max / min through the same tree (negated min as a max)
-  double m1 = mx, m2 = -mn;
+    double est[2];
+    ls_chain_estimate2(one, 0, a.kind, a.dd.nvars, a.dd.nbasis, a.dd.mono, v, exv, est);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    m1 = fmax(m1, __shfl_down_sync(0xffffffffu, m1, o));
-    m2 = fmax(m2, __shfl_down_sync(0xffffffffu, m2, o));
-  }
-  __syncthreads();
-  if ((tid & 31) == 0) {
-    tmp_s[tid >> 5] = m1;
-    tmp_s[32 + (tid >> 5)] = m2;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    for (int w = 1; w < kNestThreads / 32; ++w) {
-      m1 = fmax(m1, tmp_s[w]);
-      m2 = fmax(m2, tmp_s[32 + w]);
+    for (int h = 0; h < 2; ++h) {
+      if (h && !two) break;
+      double nv = INFINITY;
+      if (member[h]) {
+        nv = est[h] - (double)exv[h];
+        s1 += nv;
+        s2 += nv * nv;
+        mx = fmax(mx, nv);
+        mn = fmin(mn, nv);
+      }
+      net[p[h]] = nv;
     }
-    double* pb = part + (size_t)blockIdx.x * 4;
-    pb[0] = t1;
-    pb[1] = t2;
-    pb[2] = m1;
-    pb[3] = m2;
   }
-  if (!last_block(ticket, &flag_s)) return;
-  double t4[2];
-  thread_partials<2>(part, 4, gridDim.x, t4);
-  double mx4 = -INFINITY, mn4 = -INFINITY;
-  for (int b = tid; b < (int)gridDim.x; b += blockDim.x) {
-    mx4 = fmax(mx4, __ldcg(part + (size_t)b * 4 + 2));
-    mn4 = fmax(mn4, __ldcg(part + (size_t)b * 4 + 3));
+  {
+    const double sums[2] = {s1, s2}, maxima[2] = {mx, -mn};
+    block_sums<2>(sums, red_s, out_s);
+    block_maxima<2>(maxima, red_s, out_s + 2);
+    if (tid < 4) part[(size_t)blockIdx.x * 4 + tid] = out_s[tid];
   }
-  const double S1 = block_sum(t4[0], red_s), S2 = block_sum(t4[1], red_s);
-  const double MX = block_max(mx4, red_s), MN = -block_max(mn4, red_s);
-  for (int i = tid; i < (int)(sizeof(SelState) / 4); i += blockDim.x) ((unsigned*)&S)[i] = 0u;
-  __syncthreads();
-  if (tid == 0) {
-    if (d == 0 && (MX <= 0.0 || MN >= 0.0)) {
+  unsigned gen = 1;
+  bool ok = grid_wait(&sync->barrier, gen, &flag_s);
+  // every CTA joins the partials in the same order
+  {
+    double t[2], m[2] = {-INFINITY, -INFINITY};
+    thread_partials<2>(part, 4, gridDim.x, t);
+    for (int b = tid; b < (int)gridDim.x; b += kSelThreads) {
+      m[0] = fmax(m[0], __ldcg(part + (size_t)b * 4 + 2));
+      m[1] = fmax(m[1], __ldcg(part + (size_t)b * 4 + 3));
+    }
+    block_sums<2>(t, red_s, out_s);
+    block_maxima<2>(m, red_s, out_s + 2);
+    const double S1 = out_s[0], S2 = out_s[1], MX = out_s[2], MN = -out_s[3];
+    if (tid == 0) {
+      S = SelState{};
       S.phase = kPhDone;
-      stopped[e] = 1;
+      if (d > 0 || !(MX <= 0.0 || MN >= 0.0)) {
+        const int n_pre = d == 0 ? paths : npaths[row];
+        S.lo_t = (int)(n_pre * a.lower_frac);
+        S.hi_t = (int)(n_pre * a.upper_frac);
+        S.mult = a.mult;
+        if (n_pre > S.lo_t && n_pre < S.hi_t) {
+          S.phase = kPhBranch;
+        } else {
+          const double mean = S1 / n_pre;
+          S.g = sqrt(S2 / n_pre - mean * mean) * a.sds;
+          S.phase = kPhInit;
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int pass = 0; pass < kSelPasses && S.phase != kPhDone && ok; ++pass) {
+    sel_thresholds(S, thr_s);
+    const int nb = S.nb;
+    for (int i = tid; i < nb; i += kSelThreads) hist_s[i] = 0;
+    __syncthreads();
+    const double top = thr_s[nb - 1];
+    for (long long p = p_begin; p < paths; p += stride) {
+      const double x = fabs(net[p]);
+      if (!(x <= top)) continue;
+      int lo = 0, hi = nb - 1;  // first i with x <= thr[i]
+      while (lo < hi) {
+        const int m = (lo + hi) >> 1;
+        if (x <= thr_s[m])
+          hi = m;
+        else
+          lo = m + 1;
+      }
+      atomicAdd(&hist_s[lo], 1);
+    }
+    __syncthreads();
+    int* hist_g = sync->hist[pass];
+    for (int i = tid; i < nb; i += kSelThreads)
+      if (hist_s[i]) atomicAdd(hist_g + i, hist_s[i]);
+    ok = grid_wait(&sync->barrier, ++gen, &flag_s);
+    // counts = inclusive prefix of the totals (nb <= 256: eight warps)
+    static_assert(kSelBatch == 256 && kSelThreads >= kSelBatch, "one thread per bin");
+    int c = tid < nb ? __ldcg(hist_g + tid) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, c, o);
+      if (lane >= o) c += t;
+    }
+    if (lane == 31) before_s[warp] = c;
+    __syncthreads();
+    if (tid < nb) {
+      int before = 0;
+      for (int w = 0; w < warp; ++w) before += before_s[w];
+      hist_s[tid] = before + c;
+    }
+    __syncthreads();
+    if (tid == 0) sel_advance(S, thr_s, hist_s);
+    __syncthreads();
+  }
+  const bool nest = ok && S.phase == kPhDone && S.after > a.min_paths;
+  if (blockIdx.x == 0 && tid == 0) {
+    int st = S.status;
+    if (!ok)
+      st |= kSelWait;
+    else if (S.phase != kPhDone)
+      st |= kSelIncomplete;
+    if (st) atomicOr(status, st);
+    if (nest) {
+      cuts[row * 2] = -S.cut;
+      cuts[row * 2 + 1] = S.cut;
+      npaths[row + 1] = S.after;
     } else {
-      const int n_pre = d == 0 ? paths : npaths[row];
-      S.lo_t = (int)(n_pre * a.lower_frac);
-      S.hi_t = (int)(n_pre * a.upper_frac);
-      S.mult = a.mult;
-      if (n_pre > S.lo_t && n_pre < S.hi_t) {
-        S.phase = kPhBranch;
-      } else {
-        const double mean = S1 / n_pre;
-        S.g = sqrt(S2 / n_pre - mean * mean) * a.sds;
-        S.phase = kPhInit;
-      }
+      stopped[e] = 1;  // every CTA is past its read of the flag (first barrier)
     }
-    *ticket = 0u;
   }
-  __syncthreads();
-  if (S.phase != kPhDone) sel_prepare(S, tmp_s, &n_s);
-  copy_state(state, &S);
-}
-
-// One selection pass: counts of |net| <= each pending threshold, then the
-// last CTA advances the search.  When it ends: more than min_paths paths
-// selected -> cuts of regression d and the path count of regression d + 1;
-// otherwise the date stops nesting.
-__global__ void __launch_bounds__(kNestThreads)
-    nested_select_kernel(const __grid_constant__ NestArgs a, const double* __restrict__ net,
-                         int* __restrict__ hist_g, unsigned int* __restrict__ ticket,
-                         int* __restrict__ stopped, SelState* __restrict__ state,
-                         double* __restrict__ cuts, int* __restrict__ npaths,
-                         int* __restrict__ status) {
-  __shared__ double thr_s[kSelBatch];
-  __shared__ int hist_s[kSelBatch];
-  __shared__ SelState S;
-  __shared__ double tmp_s[kSelBatch];
-  __shared__ int flag_s, n_s, done_s;
-  const int e = a.e, tid = threadIdx.x;
-  if (stopped[e]) return;
-  const int phase = state->phase, nb = state->nb;
-  if (phase == kPhDone) return;
-  for (int i = tid; i < kSelBatch; i += blockDim.x) {
-    thr_s[i] = i < nb ? state->thr[i] : 0.0;
-    hist_s[i] = 0;
-  }
-  __syncthreads();
-  const double top = thr_s[nb - 1];
-  for (int p = blockIdx.x * blockDim.x + tid; p < a.paths; p += gridDim.x * blockDim.x) {
-    const double x = fabs(net[p]);
-    if (!(x <= top)) continue;
-    int lo = 0, hi = nb - 1;  // first i with x <= thr[i]
-    while (lo < hi) {
-      const int m = (lo + hi) >> 1;
-      if (x <= thr_s[m])
-        hi = m;
-      else
-        lo = m + 1;
-    }
-    atomicAdd(&hist_s[lo], 1);
-  }
-  __syncthreads();
-  // integer counts: the totals do not depend on the order of the adds
-  for (int i = tid; i < nb; i += blockDim.x)
-    if (hist_s[i]) atomicAdd(hist_g + i, hist_s[i]);
-  if (!last_block(ticket, &flag_s)) return;
-  for (int i = tid; i < nb; i += blockDim.x) {
-    hist_s[i] = __ldcg(hist_g + i);
-    hist_g[i] = 0;  // zero for the next pass
-  }
-  copy_state(&S, state);
-  __syncthreads();
-  if (tid == 0) {
-    int run = 0;
-    for (int i = 0; i < nb; ++i) {
-      run += hist_s[i];
-      S.cnt[i] = run;
-    }
-    const bool done = sel_run(S);
-    const size_t row = (size_t)e * a.rows + a.d;
-    if (done) {
-      if (S.after > a.min_paths) {
-        cuts[row * 2] = -S.cut;
-        cuts[row * 2 + 1] = S.cut;
-        npaths[row + 1] = S.after;
-      } else {
-        stopped[e] = 1;
-      }
-    } else if (a.last) {
-      S.status |= kSelIncomplete;
-      S.phase = kPhDone;
-      stopped[e] = 1;
-    }
-    if (S.status) atomicOr(status, S.status);
-    done_s = (S.phase == kPhDone);
-    *ticket = 0u;
-  }
-  __syncthreads();
-  if (!done_s) sel_prepare(S, tmp_s, &n_s);
-  copy_state(state, &S);
-}
-
-// Moments of the basis variables over the paths of regression d (|net| <=
-// cut of d - 1): means / sds row e * rows + d (GenerateLSRegressionMatrix
-// SelectivelyNormalisingVariables_gold, gold/LS_regression.h:524-600).
-__global__ void __launch_bounds__(kNestThreads)
-    nested_moments_kernel(const __grid_constant__ NestArgs a, const float* __restrict__ vars,
-                          const double* __restrict__ net, const double* __restrict__ cuts,
-                          const int* __restrict__ npaths, double* __restrict__ part,
-                          unsigned int* __restrict__ ticket, const int* __restrict__ stopped,
-                          float* __restrict__ means, float* __restrict__ sds) {
-  __shared__ double red_s[kNestThreads / 32];
-  __shared__ int flag_s;
-  const int e = a.e, tid = threadIdx.x;
-  if (stopped[e]) return;
-  const size_t row = (size_t)e * a.rows + a.d;
-  const double cut = cuts[(row - 1) * 2 + 1];
+  if (!nest || !means) return;
+  const double cut = S.cut;
   double acc[2 * kMaxVars] = {0, 0, 0, 0, 0, 0};
-  for (int p = blockIdx.x * blockDim.x + tid; p < a.paths; p += gridDim.x * blockDim.x) {
+  for (long long p = p_begin; p < paths; p += stride) {
     if (!(fabs(net[p]) <= cut)) continue;
 #pragma unroll
     for (int v = 0; v < kMaxVars; ++v) {
-      const double x = v < a.dd.nvars ? vars[((size_t)e * kMaxVars + v) * a.paths + p] : 0.0;
+      const double x = v < a.dd.nvars ? vars[((size_t)e * kMaxVars + v) * paths + p] : 0.0;
       acc[2 * v] += x;
       acc[2 * v + 1] += x * x;
     }
   }
-#pragma unroll
-  for (int i = 0; i < 2 * kMaxVars; ++i) {
-    const double t = block_sum(acc[i], red_s);
-    if (tid == 0) part[(size_t)blockIdx.x * 8 + i] = t;
-  }
-  if (!last_block(ticket, &flag_s)) return;
+  // every CTA has read the net partials before the second barrier at the
+  // latest (a search takes one pass or more), so their buffer is free
+  block_sums<2 * kMaxVars>(acc, red_s, out_s);
+  if (tid < 2 * kMaxVars) part[(size_t)blockIdx.x * 8 + tid] = out_s[tid];
+  if (!last_block(&sync->ticket, &flag_s)) return;
   double t6[2 * kMaxVars];
   thread_partials<2 * kMaxVars>(part, 8, gridDim.x, t6);
-#pragma unroll
-  for (int v = 0; v < kMaxVars; ++v) {
-    const double s1 = block_sum(t6[2 * v], red_s);
-    const double s2 = block_sum(t6[2 * v + 1], red_s);
-    if (tid == 0) {
-      double m = 0.0, sd = 1.0;
-      if (v < a.dd.nvars) {
-        const double n = (double)npaths[row];
-        m = s1 / n;
-        const double var = s2 / n - m * m;
-        sd = var > 0.0 ? sqrt(var) : 1.0;
-      }
-      means[row * kMaxVars + v] = (float)m;
-      sds[row * kMaxVars + v] = (float)sd;
+  block_sums<2 * kMaxVars>(t6, red_s, out_s);
+  if (tid < kMaxVars) {
+    double m = 0.0, sd = 1.0;
+    if (tid < a.dd.nvars) {
+      const double n = (double)S.after;
+      m = out_s[2 * tid] / n;
+      const double var = out_s[2 * tid + 1] / n - m * m;
+      sd = var > 0.0 ? sqrt(var) : 1.0;
     }
+    means[(row + 1) * kMaxVars + tid] = (float)m;
+    sds[(row + 1) * kMaxVars + tid] = (float)sd;
   }
-  if (tid == 0) *ticket = 0u;
 }
 
 // Path counts: regression 0 of every date uses all paths; the rest start
@@ -657,23 +624,13 @@ struct NestWs {
   double* red;           // final reduction
   double* net;           // [P]
   double* npart;         // net / moments partials: blocks x 8
-  int* hist;             // selection histogram [kSelBatch], zero between passes
-  unsigned int* tickets; // [4]
-  SelState* state;
+  NestSync* sync;        // [2]
   int* stopped;          // [E]
   int* npaths;           // [E][kMaxDepth]
 };
 
-// CTAs of the net, selection and moments passes: up to kNestCtasPerSm per
-// SM, enough warps in flight for these latency-bound streaming passes.
-constexpr int kNestCtasPerSm = 8;
-int nest_grid(int paths) {
-  return std::max(1, std::min(div_up(paths, kNestThreads), kNestCtasPerSm * ls_gram_blocks()));
-}
-
 size_t nested_ws_bytes(int paths, int n_ex, NestWs* w, char* base) {
   const size_t nb = (size_t)ls_gram_blocks();
-  const size_t ng = (size_t)kNestCtasPerSm * nb;
   size_t off = 0;
   auto take = [&](size_t bytes) {
     char* p = base ? base + off : nullptr;
@@ -687,14 +644,28 @@ size_t nested_ws_bytes(int paths, int n_ex, NestWs* w, char* base) {
   t.mom = (double*)take((size_t)n_ex * nb * 6 * sizeof(double));
   t.red = (double*)take(512 * sizeof(double));
   t.net = (double*)take((size_t)paths * sizeof(double));
-  t.npart = (double*)take(ng * 8 * sizeof(double));
-  t.hist = (int*)take(kSelBatch * sizeof(int));
-  t.tickets = (unsigned int*)take(4 * sizeof(unsigned int));
-  t.state = (SelState*)take(sizeof(SelState));
+  t.npart = (double*)take(nb * 8 * sizeof(double));
+  t.sync = (NestSync*)take(2 * sizeof(NestSync));
   t.stopped = (int*)take((size_t)n_ex * sizeof(int));
   t.npaths = (int*)take((size_t)n_ex * kMaxDepth * sizeof(int));
   if (w) *w = t;
   return off + 256;
+}
+
+// The selection kernel as a cooperative launch (its CTAs wait on one
+// another); `k` counts the regression's selection launches.
+int launch_select(NestArgs a, int grid, const float* vars, const float* ex, const double* beta,
+                  float* means, float* sds, double* cuts, int* npaths, const NestWs& w, int k,
+                  int* status, cudaStream_t s) {
+  double *net = w.net, *part = w.npart;
+  NestSync *sync = w.sync + (k & 1), *next = w.sync + ((k + 1) & 1);
+  int* stopped = w.stopped;
+  void* args[] = {&a,      &vars, &ex,   &beta, &means, &sds,    &cuts,
+                  &npaths, &net,  &part, &sync, &next,  &stopped, &status};
+  TRY(check_cuda(cudaLaunchCooperativeKernel((const void*)nested_select_kernel, dim3(grid),
+                                             dim3(kSelThreads), args, 0, s),
+                 "nested_select_kernel"));
+  return check_launch("nested_select_kernel");
 }
 
 }  // namespace
@@ -744,8 +715,7 @@ extern "C" int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_v
   TRY(check_cuda(cudaMemsetAsync(d_status, 0, sizeof(int), s), "nested: status"));
   TRY(check_cuda(cudaMemsetAsync(w.counter, 0, (size_t)n_exercise * sizeof(unsigned int), s),
                  "nested: counters"));
-  TRY(check_cuda(cudaMemsetAsync(w.tickets, 0, 4 * sizeof(unsigned int), s), "nested: tickets"));
-  TRY(check_cuda(cudaMemsetAsync(w.hist, 0, kSelBatch * sizeof(int), s), "nested: histogram"));
+  TRY(check_cuda(cudaMemsetAsync(w.sync, 0, 2 * sizeof(NestSync), s), "nested: histograms"));
   TRY(check_cuda(cudaMemsetAsync(w.stopped, 0, (size_t)n_exercise * sizeof(int), s),
                  "nested: flags"));
   TRY(check_cuda(cudaMemsetAsync(d_cuts, 0, rows * 2 * sizeof(double), s), "nested: cuts"));
@@ -764,12 +734,13 @@ extern "C" int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_v
   }
   const int nblk = ls_gram_blocks();
   const int grid_path = grid_for(paths, kNestThreads, 4);
-  const int grid_nest = nest_grid(paths);
+  const int grid_sel = std::min(div_up(paths, kSelThreads), nblk);
+  int launches = 0;
   const LsRuleView rule{D, d_beta, means, sds, D > 1 ? d_cuts : nullptr, nullptr};
   for (int e = n_exercise - 1; e >= 0; --e) {
     if (e + 1 < n_exercise) {
       nested_decide_kernel<<<grid_path, kNestThreads, 0, s>>>(
-          dates[e + 1], e + 1, 1, rule, d_vars, d_cf, d_ex, d_num, w.y, paths);
+          dates[e + 1], ls_basis_kind(dates[e + 1]), e + 1, 1, rule, d_vars, d_cf, d_ex, d_num, w.y, paths);
       TRY(check_launch("nested_decide_kernel"));
     }
     const int slots = dates[e].nbasis + 1;
@@ -779,6 +750,7 @@ extern "C" int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_v
       NestArgs a;
       memset(&a, 0, sizeof(a));
       a.dd = dates[e];
+      a.kind = ls_basis_kind(dates[e]);
       a.e = e;
       a.rows = D;
       a.paths = paths;
@@ -788,26 +760,12 @@ extern "C" int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_v
       a.sds = sel->sds;
       a.mult = sel->multiplier;
       if (d > 0) {
-        // net values of regression d - 1, then the search for its cuts
+        // net values of regression d - 1, the search for its cuts, and the
+        // moments of regression d's paths
         a.d = d - 1;
-        nested_net_kernel<<<grid_nest, kNestThreads, 0, s>>>(
-            a, d_vars, d_ex, d_beta, means, sds, d_cuts, npaths, w.net, w.npart, w.tickets + 0,
-            w.stopped, w.state);
-        TRY(check_launch("nested_net_kernel"));
-        for (int pass = 0; pass < kSelPasses; ++pass) {
-          a.last = pass + 1 == kSelPasses;
-          nested_select_kernel<<<grid_nest, kNestThreads, 0, s>>>(
-              a, w.net, w.hist, w.tickets + 1, w.stopped, w.state, d_cuts, npaths, d_status);
-          TRY(check_launch("nested_select_kernel"));
-        }
-        a.d = d;
-        a.last = 0;
-        if (normalise) {
-          nested_moments_kernel<<<grid_nest, kNestThreads, 0, s>>>(
-              a, d_vars, w.net, d_cuts, npaths, w.npart, w.tickets + 2, w.stopped, d_means,
-              d_sds);
-          TRY(check_launch("nested_moments_kernel"));
-        }
+        TRY(launch_select(a, grid_sel, d_vars, d_ex, d_beta, normalise ? d_means : nullptr,
+                          normalise ? d_sds : nullptr, d_cuts, npaths, w, launches++, d_status,
+                          s));
       }
       LSDateParams P;
       memset(&P, 0, sizeof(P));
@@ -828,7 +786,7 @@ extern "C" int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_v
                       w.counter, nullptr, d_status, nullptr, s));
     }
   }
-  nested_decide_kernel<<<grid_path, kNestThreads, 0, s>>>(dates[0], 0, 0, rule, d_vars, d_cf,
+  nested_decide_kernel<<<grid_path, kNestThreads, 0, s>>>(dates[0], ls_basis_kind(dates[0]), 0, 0, rule, d_vars, d_cf,
                                                           d_ex, d_num, w.y, paths);
   TRY(check_launch("nested_decide_kernel"));
   return reduce_launch(w.y, d_num, (size_t)paths, 1.0 / (double)paths, w.red, d_price, s);

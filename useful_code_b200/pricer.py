@@ -270,7 +270,7 @@ class Pipeline:
     def regress_nested_graph(self, ls: LSInputs, select: Selector):
         """lmm_ls_regress_nested on these inputs captured as a CUDA graph.
 
-        The entry point issues a fixed sequence of launches (about 2,300 at
+        The entry point issues a fixed sequence of launches (about 640 at
         80 dates and depth 4) with no host synchronisation, so it captures
         whole; ``graph.replay()`` recomputes the rule from the current
         contents of ``ls`` into the returned result's buffers, without the
