@@ -409,7 +409,8 @@ int lmm_step_to_exercise_indices(const int* h_gen_indices, int n_gen,
  * normalise != 0; means/sds are then written).  d_cf and d_ex ([E][P],
  * deflated to the exercise time) may be NULL.  Outputs: d_beta[E][16]
  * (FP64), optional d_gram[E][16][17] (normalised Gram | target column),
- * d_status (bit 1: zero Gram, 2: Cholesky failed, 4: jitter used) and
+ * d_status (bit 1: zero Gram, 2: Cholesky failed, 4: jitter used, 32: a
+ * bounded wait between the launch's CTAs ran out) and
  * d_price = mean_p y_p / N_0(p).  Workspace: lmm_ls_workspace_bytes(). */
 size_t lmm_ls_workspace_bytes(int paths, int n_exercise);
 int lmm_ls_regress(int n_exercise, int paths, const float* d_vars,

@@ -16,15 +16,19 @@
 //                        exponent tables, one table per exercise date
 //   in-sample price      mean_p y_p / N_0(p)  (MultiLS_regression.cpp:407-416)
 // The reference solves each normal-equation system on the host by SVD after
-// a device-to-host copy (LinearSolverConcrete_main.cu:127-188); here each
-// date is one kernel: the Gram sums stay on the device and the last CTA of
-// the launch solves them with a warp-parallel FP64 Cholesky, so the loop is
-// launch-only (one launch per date) and can be captured in a graph.
+// a device-to-host copy (LinearSolverConcrete_main.cu:127-188); here the
+// Gram sums stay on the device and are solved there by a warp-parallel FP64
+// Cholesky, so the loop is launch-only and can be captured in a graph: one
+// cooperative launch for the whole loop (ls_run_kernel), or one launch per
+// date (ls_date_kernel; tables of more than 11 slots, nested regressions and
+// the sharded protocol).
 #include "lmm_common.cuh"
 #include "lmm_device.cuh"
 #include "ls_common.cuh"
 
+#include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 using namespace lmm;
@@ -623,6 +627,282 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
   }
 }
 
+// ---------------------------------------------------------------------------
+// The whole backward loop (depth 1) as one cooperative launch.
+//
+// Per date the work is that of ls_date_kernel; what the separate launches
+// cost on top is the gap between two launches, the cold start of the input
+// pipeline, and the serial tail (CTA partials, their sum, the solve) during
+// which nothing else runs.  Here every CTA keeps its paths for all dates: it
+// issues the next date's first input copies before it waits for the other
+// CTAs, every CTA sums the partials and solves for itself (the same
+// arithmetic in the same order, so all hold the same coefficients, with no
+// second exchange).
+// The dates with few functions (the last ones, with fewer variables) run as
+// ls_date_kernel's instantiation for them does, with the same order of the
+// partials: their Grams are close to singular, and their coefficients would
+// show another order of the sums.  The coefficients are those of one launch
+// per date to the last bit.
+//
+// For tables of at most 11 slots, whose rows one warp holds.  80 dates, 10
+// functions: 2.85 -> 2.19 ms at 2^20 paths, 1.97 -> 1.33 at 2^18; 40 dates, 6
+// functions: 0.70 -> 0.41 ms at 2^16, 0.62 -> 0.39 at 4,099.  Larger tables
+// keep one launch per date: with their rows split over warp pairs the loop
+// gained less (120 dates, 12 functions, 2.65 against 3.0 ms at 150,001 paths),
+// and there the compiler contracts other products into the sums than in
+// ls_date_kernel, which the third powers' Grams turn into 1e-3 of a
+// coefficient.
+// ---------------------------------------------------------------------------
+struct LSRun {
+  int n_ex, paths, vec16;
+  unsigned char known[kMaxSteps];  // the date's table is the launch's KIND
+  LSDate date[kMaxSteps];
+};
+
+constexpr int kLsWait = 32;  // status: a wait of the grid ran out
+
+template <int KR, int KIND>
+__global__ void __launch_bounds__(LsThreads<KR>::value, 1)
+    ls_run_kernel(const __grid_constant__ LSRun R, const float* __restrict__ vars,
+                  const float* __restrict__ means, const float* __restrict__ sds,
+                  const float* __restrict__ cf, const float* __restrict__ ex,
+                  const float* __restrict__ num, double* __restrict__ beta, float* y,
+                  double* part0, double* part1, unsigned int* counter,
+                  double* __restrict__ gram_out, int* __restrict__ status) {
+  constexpr int NPAIRS = KR * (KR + 1) / 2;  // row of a CTA's partials
+  constexpr int T = LsThreads<KR>::value;
+  constexpr int NW = T / 32;
+  __shared__ double beta_s[kMaxBasis];           // coefficients of the date solved last
+  __shared__ float mom_s[kMaxSteps][2][kMaxVars];  // mean and 1 / sd per date
+  __shared__ double red_s[NW][NPAIRS];
+  __shared__ double share_s[T];
+  __shared__ double sums_s[NPAIRS];
+  __shared__ double G_s[kLsMaxSlots * kLsMaxSlots];
+  __shared__ int ok_s;
+  extern __shared__ float ls_stage[];  // [kLsStages][kLsInputs][T]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int paths = R.paths, E = R.n_ex;
+  if (means)
+    for (int i = tid; i < E * kMaxVars; i += T) {
+      mom_s[i / kMaxVars][0][i % kMaxVars] = means[i];
+      mom_s[i / kMaxVars][1][i % kMaxVars] = 1.0f / sds[i];
+    }
+  const int r0 = lane >> 3, c4 = (lane & 7) * 4;
+  float* const wstage = ls_stage + warp * 32;
+  const int w0 = blockIdx.x * T + warp * 32, stride = gridDim.x * T;
+  // input row i of date e's loop (null: not read)
+  auto row_ptr = [&](int e, int i) -> const float* {
+    const size_t cur = (size_t)e * paths, nxt = cur + paths;
+    if (i < kInCf)
+      return i < R.date[e].nvars ? vars + ((size_t)e * kMaxVars + i) * paths : nullptr;
+    if (i == kInCf) return cf ? cf + cur : nullptr;
+    if (e + 1 >= E) return nullptr;
+    if (i == kInY) return y;
+    if (i < kInCfNext) {
+      const int v = i - kInXNext;
+      return v < R.date[e + 1].nvars ? vars + ((size_t)(e + 1) * kMaxVars + v) * paths : nullptr;
+    }
+    if (i == kInCfNext) return cf ? cf + nxt : nullptr;
+    if (i == kInExNext) return ex ? ex + nxt : nullptr;
+    return i == kInNum ? num + cur : num + nxt;
+  };
+  const float *rp0 = nullptr, *rp1 = nullptr, *rp2 = nullptr;
+  // copies the inputs of the warp's paths qw .. qw + 31 into stage it
+  // (16-byte chunks of rows r0, r0 + 4, r0 + 8 per lane when every row is
+  // aligned, else each lane its own path's values)
+  auto issue = [&](int e, int it, int qw) {
+    float* dst = wstage + (it & (kLsStages - 1)) * kLsInputs * T;
+    if (R.vec16) {
+      const int qb = qw + c4;
+      if (qb < paths) {
+        if (rp0) cp_async16(dst + r0 * T + c4, rp0 + qb);
+        if (rp1) cp_async16(dst + (r0 + 4) * T + c4, rp1 + qb);
+        if (rp2) cp_async16(dst + (r0 + 8) * T + c4, rp2 + qb);
+      }
+    } else if (qw + lane < paths) {
+#pragma unroll 1
+      for (int i = 0; i < kLsInputs; ++i) {
+        const float* rp = row_ptr(e, i);
+        if (rp) cp_async4(dst + i * T + lane, rp + qw + lane);
+      }
+    }
+    cp_async_commit();
+  };
+  auto start_date = [&](int e) {
+    if (R.vec16) {
+      rp0 = row_ptr(e, r0);
+      rp1 = row_ptr(e, r0 + 4);
+      rp2 = row_ptr(e, r0 + 8);
+    }
+#pragma unroll
+    for (int k = 0; k < kLsStages - 1; ++k) issue(e, k, w0 + k * stride);
+  };
+  // date e with KRD slots: false when a wait ran out
+  auto run_date = [&](auto kr_tag, auto kind_tag, const int e) -> bool {
+    constexpr int KRD = decltype(kr_tag)::value, KD = decltype(kind_tag)::value;
+    constexpr int NP = KRD * (KRD + 1) / 2;
+    const LSDate& cur = R.date[e];
+    const LSDate& prev = R.date[e + 1 < E ? e + 1 : e];
+    const bool has_prev = e + 1 < E;
+    const bool prev_known = has_prev && R.known[e + 1];
+    const int K = cur.nbasis, nb = gridDim.x;
+    float acc[NP];
+#pragma unroll
+    for (int q = 0; q < NP; ++q) acc[q] = 0.0f;
+    int it = 0;
+    for (int qw = w0; qw < paths; qw += stride, ++it) {
+      issue(e, it + kLsStages - 1, qw + (kLsStages - 1) * stride);
+      cp_async_wait<kLsStages - 1>();
+      __syncwarp();
+      const int p = qw + lane;
+      if (p < paths) {
+        const float* in = wstage + (it & (kLsStages - 1)) * kLsInputs * T + lane;
+        float yp = 0.0f;
+        if (has_prev) {
+          float xp[kMaxVars];
+#pragma unroll
+          for (int v = 0; v < kMaxVars; ++v)
+            xp[v] = v < prev.nvars ? in[(kInXNext + v) * T] : 0.0f;
+          const float* mean_p = means ? mom_s[e + 1][0] : nullptr;
+          const float cfn = cf ? in[kInCfNext * T] : 0.0f, exn = ex ? in[kInExNext * T] : 0.0f;
+          if (KIND != kBasisGeneric && prev_known)
+            yp = decide_values<KIND>(prev, 1, xp, mean_p, mom_s[e + 1][1], cfn, exn,
+                                     in[kInNum * T], in[kInNumNext * T], beta_s, in[kInY * T]);
+          else
+            yp = decide_values<kBasisGeneric>(prev, 1, xp, mean_p, mom_s[e + 1][1], cfn, exn,
+                                              in[kInNum * T], in[kInNumNext * T], beta_s,
+                                              in[kInY * T]);
+        }
+        y[p] = yp;
+        float x[kMaxVars];
+#pragma unroll
+        for (int v = 0; v < kMaxVars; ++v) {
+          float xv = 0.0f;
+          if (v < cur.nvars) {
+            xv = in[(kInX + v) * T];
+            if (means) xv = (xv - mom_s[e][0][v]) * mom_s[e][1][v];
+          }
+          x[v] = xv;
+        }
+        float pw[kMaxVars][3];
+        ls_powers(x, pw);
+        float phi[KRD];
+#pragma unroll
+        for (int k = 0; k < KRD - 1; ++k)
+          phi[k] = (k < (KD ? basis_K(KD) : K)) ? ls_basis<KD>(pw, cur, k) : 0.0f;
+        phi[KRD - 1] = (cf ? in[kInCf * T] : 0.0f) + yp;
+        accumulate_rows<KRD, 0, KRD>(phi, acc);
+      }
+      // every lane's reads of this stage precede its refill, issued by
+      // other lanes in a later iteration
+      __syncwarp();
+    }
+    cp_async_wait<0>();
+    int first, count;
+    warp_sums<NP>(acc, first, count);
+#pragma unroll
+    for (int i = 0; i < warp_sums_left<NP>(); ++i)
+      if (i < count) red_s[warp][first + i] = (double)acc[i];
+    __syncthreads();
+    double* part = ((E - 1 - e) & 1) ? part1 : part0;
+    for (int q = tid; q < NP; q += T) {
+      double s = 0.0;
+      for (int w = 0; w < NW; ++w) s += red_s[w][q];
+      part[(size_t)blockIdx.x * NPAIRS + q] = s;
+    }
+    // the next date's first inputs (all warps' stores of y precede the
+    // barrier above) while the other CTAs finish
+    if (e > 0) start_date(e - 1);
+    __syncthreads();
+    if (tid == 0) {
+      const unsigned want = (unsigned)(E - e) * gridDim.x;
+      __threadfence();
+      atomicAdd(counter, 1u);
+      int ok = 0;
+      for (int i = 0; i < (1 << 22) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
+      __threadfence();
+      ok_s = ok;
+    }
+    __syncthreads();
+    if (!ok_s) return false;  // never while every CTA is resident
+    // thread (sub, q) adds every tpq-th CTA's partial of pair q; the shares of
+    // a pair follow in a fixed order
+    {
+      constexpr int tpq = T / NP;
+      const int sub = tid / NP, q = tid - sub * NP;
+      double v = 0.0;
+      if (sub < tpq) {
+        const double* src = part + q;
+#pragma unroll 11
+        for (int b = sub; b < nb; b += tpq) v += __ldcg(src + (size_t)b * NPAIRS);
+      }
+      share_s[tid] = v;
+      __syncthreads();
+      if (tid < NP) {
+        double t = 0.0;
+        for (int k = 0; k < tpq; ++k) t += share_s[k * NP + tid];
+        sums_s[tid] = t / (double)paths;
+      }
+      __syncthreads();
+    }
+    // G_s[i][j] (i, j < K) and the right-hand side in column kLsMaxSlots - 1
+    for (int idx = tid; idx < kLsMaxSlots * kLsMaxSlots; idx += T) {
+      const int i = idx / kLsMaxSlots, j = idx - i * kLsMaxSlots;
+      double v = 0.0;
+      if (i < K && j < K) {
+        const int a = i > j ? i : j, b = i > j ? j : i;
+        v = sums_s[a * (a + 1) / 2 + b];
+      } else if (i < K && j == kLsMaxSlots - 1) {
+        v = sums_s[(KRD - 1) * KRD / 2 + i];
+      }
+      G_s[idx] = v;
+    }
+    __syncthreads();
+    if (warp == 0) {
+      const int st = warp_cholesky_solve<basis_K(KD)>(G_s, K, beta_s, share_s);
+      if (lane == 0 && st && blockIdx.x == 0) atomicOr(status, st);
+    }
+    __syncthreads();
+    if (blockIdx.x == 0) {
+      if (tid < kMaxBasis) beta[(size_t)e * kMaxBasis + tid] = beta_s[tid];
+      if (gram_out) {
+        double* g = gram_out + (size_t)e * kMaxBasis * (kMaxBasis + 1);
+        for (int idx = tid; idx < K * (kMaxBasis + 1); idx += T) {
+          const int i = idx / (kMaxBasis + 1), j = idx - i * (kMaxBasis + 1);
+          double v = 0.0;
+          if (j < K)
+            v = G_s[i * kLsMaxSlots + j];
+          else if (j == K)
+            v = G_s[i * kLsMaxSlots + kLsMaxSlots - 1];
+          g[idx] = v;
+        }
+        __syncthreads();  // before the next date's G_s
+      }
+    }
+    return true;
+  };
+  start_date(E - 1);
+  __syncthreads();
+  for (int e = E - 1; e >= 0; --e) {
+    bool ok;
+    // the compile-time table where the date and the next (whose decision it
+    // applies) both have it, as launch_date chooses
+    if (KIND != kBasisGeneric && R.known[e] && (e + 1 == E || R.known[e + 1]))
+      ok = run_date(std::integral_constant<int, KR>(), std::integral_constant<int, KIND>(), e);
+    else if (KR > 7 && R.date[e].nbasis < 7)
+      ok = run_date(std::integral_constant<int, 7>(),
+                    std::integral_constant<int, kBasisGeneric>(), e);
+    else
+      ok = run_date(std::integral_constant<int, KR>(),
+                    std::integral_constant<int, kBasisGeneric>(), e);
+    if (!ok) {
+      if (tid == 0) atomicOr(status, kLsWait);
+      cp_async_wait<0>();
+      return;
+    }
+  }
+}
+
 // Final decision at date 0 (no deflation): y holds the value at date 0.
 __global__ void ls_final_kernel(const __grid_constant__ LSDateParams P,
                                 const float* __restrict__ vars,
@@ -839,6 +1119,52 @@ int launch_date(const LSDateParams& P_in, int grid, const float* vars,
   return check_launch("ls_date_kernel");
 }
 
+// The whole backward loop (ls_run_kernel), instantiated for the most slots
+// of any date and for the table that most dates share; -1 (nothing launched)
+// for tables of more than 11 slots.  `part` holds nblk x kLsMaxPairs doubles,
+// room for two buffers of 66.
+int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const float* sds,
+               const float* cf, const float* ex, const float* num, double* beta, float* y,
+               double* part, unsigned int* counter, double* gram, int* status,
+               cudaStream_t s) {
+  auto al16 = [](const void* q) { return ((uintptr_t)q & 15u) == 0; };
+  R.vec16 = (R.paths % 4 == 0) && al16(vars) && al16(cf) && al16(ex) && al16(num) && al16(y);
+  int slots = 0, votes[5] = {0, 0, 0, 0, 0}, kind = kBasisGeneric;
+  for (int e = 0; e < R.n_ex; ++e) {
+    slots = std::max(slots, R.date[e].nbasis + 1);
+    ++votes[ls_basis_kind(R.date[e])];
+  }
+  if (slots > 11) return -1;
+  for (int k : {kBasisC2, kBasisQuad, kBasisCross})
+    if (votes[k] && (kind == kBasisGeneric || votes[k] > votes[kind])) kind = k;
+  if (kind == kBasisC2 && slots > 7) kind = kBasisGeneric;
+  for (int e = 0; e < R.n_ex; ++e)
+    R.known[e] = kind != kBasisGeneric && ls_basis_kind(R.date[e]) == kind;
+  auto go = [&](auto kern, int pairs, size_t stage, int threads) -> int {
+    double* part1 = part + (size_t)nblk * pairs;
+    int st = ls_stage_attr(kern, stage);
+    if (st) return st;
+    const int grid = std::min(div_up(R.paths, threads), nblk);
+    void* args[] = {&R, &vars, &means, &sds, &cf, &ex, &num, &beta, &y, &part, &part1,
+                    &counter, &gram, &status};
+    st = check_cuda(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(threads),
+                                                args, stage, s),
+                    "ls_run_kernel");
+    return st ? st : check_launch("ls_run_kernel");
+  };
+#define LMM_LS_RUN(KR, KIND)                                                            \
+  go(ls_run_kernel<KR, KIND>, KR*(KR + 1) / 2, ls_stage_bytes<KR, 1, false>(),          \
+     LsThreads<KR>::value)
+  switch (kind) {
+    case kBasisC2: return LMM_LS_RUN(7, kBasisC2);
+    case kBasisQuad: return LMM_LS_RUN(11, kBasisQuad);
+    case kBasisCross: return LMM_LS_RUN(11, kBasisCross);
+    default: break;
+  }
+  return slots <= 7 ? LMM_LS_RUN(7, kBasisGeneric) : LMM_LS_RUN(11, kBasisGeneric);
+#undef LMM_LS_RUN
+}
+
 }  // namespace lmm
 
 extern "C" size_t lmm_ls_workspace_bytes(int paths, int n_exercise) {
@@ -892,25 +1218,33 @@ extern "C" int lmm_ls_regress(int n_exercise, int paths, const float* d_vars,
   st = check_cuda(cudaMemsetAsync(counter, 0, (size_t)n_exercise * sizeof(unsigned int), s),
                   "lmm_ls_regress: counter reset");
   if (st) return st;
-  for (int e = n_exercise - 1; e >= 0; --e) {
+  LSRun run;
+  memset(&run, 0, sizeof(run));
+  run.n_ex = n_exercise;
+  run.paths = paths;
+  for (int e = 0; e < n_exercise; ++e) {
+    st = ls_fill_date(spec, e, &run.date[e]);
+    if (st) return st;
+  }
+  st = launch_run(run, nblk, d_vars, means, sds, d_cf, d_ex, d_num, d_beta, y, part, counter,
+                  d_gram, d_status, s);
+  if (st > 0) return st;
+  // tables of more than 11 slots: one launch per date
+  for (int e = n_exercise - 1; st < 0 && e >= 0; --e) {
     LSDateParams P;
     memset(&P, 0, sizeof(P));
     P.e = e;
     P.paths = paths;
-    st = ls_fill_date(spec, e, &P.cur);
-    if (st) return st;
+    P.cur = run.date[e];
     P.has_prev = (e + 1 < n_exercise);
-    if (P.has_prev) {
-      st = ls_fill_date(spec, e + 1, &P.prev);
-      if (st) return st;
-    }
+    if (P.has_prev) P.prev = run.date[e + 1];
     const int slots = P.cur.nbasis + 1;
     const int per_cta = slots <= 11 ? 512 : slots <= 13 ? 256 : 192;
     int grid = div_up(paths, per_cta);
     if (grid > nblk) grid = nblk;
-    st = launch_date(P, grid, d_vars, means, sds, d_cf, d_ex, d_num, d_beta, y,
-                     part, counter, d_gram, d_status, nullptr, s);
-    if (st) return st;
+    const int one = launch_date(P, grid, d_vars, means, sds, d_cf, d_ex, d_num, d_beta, y,
+                                part, counter, d_gram, d_status, nullptr, s);
+    if (one) return one;
   }
   LSDateParams P;
   memset(&P, 0, sizeof(P));
