@@ -112,54 +112,100 @@ __device__ __forceinline__ float icdf_sb_fast(uint32_t vi) {
   return sgn * ((z * pq.x) * rcp_ftz(pq.y));
 }
 
+// icdf_sb_fast for two points per thread, each half with icdf_sb_fast's own
+// roundings: the numerator and denominator recurrences run on the pair of
+// points (no packing of a point's own numerator and denominator), and the
+// sign, +1 for integers from 2^31, is set as a bit.
+__device__ __forceinline__ float2 icdf_sb_fast2(uint32_t va, uint32_t vb) {
+  auto tail = [](uint32_t v) {
+    return fmaxf(__uint2float_rn(min(v, 0u - v)) * 4.656612873077392578125e-10f,
+                 2.3283064365386963e-10f);
+  };
+  const float2 z = make_float2(-log_ftz(tail(va)), -log_ftz(tail(vb)));
+  float2 p = __ffma2_rn(dup2(4.744820732427972462e-6f), z, dup2(0.0020751409553756572917f));
+  float2 q = __ffma2_rn(dup2(0.00010590620919921025259f), z, dup2(0.0120098270559197768f));
+  p = __ffma2_rn(p, z, dup2(0.087403248265958578062f));
+  q = __ffma2_rn(q, z, dup2(0.23668431621373705623f));
+  p = __ffma2_rn(p, z, dup2(0.80002295072483916762f));
+  q = __ffma2_rn(q, z, dup2(1.2499328117341603014f));
+  p = __ffma2_rn(p, z, dup2(1.9797154223229267471f));
+  q = __ffma2_rn(q, z, dup2(2.0795584360534589311f));
+  p = __ffma2_rn(p, z, dup2(1.2533136835212087879f));
+  q = __ffma2_rn(q, z, dup2(1.0f));
+  const float2 x = __fmul2_rn(__fmul2_rn(z, p), make_float2(rcp_ftz(q.x), rcp_ftz(q.y)));
+  return make_float2(__uint_as_float(__float_as_uint(x.x) ^ (~va & 0x80000000u)),
+                     __uint_as_float(__float_as_uint(x.y) ^ (~vb & 0x80000000u)));
+}
+
 // ---------------------------------------------------------------------------
 // Fused variates: Sobol point -> XOR scramble -> inverse normal -> bridge.
-// One thread per (path, factor), one CTA per 128 consecutive paths and one
-// factor.  With n = first_index + p and gray(n) = n ^ (n >> 1), the bits of
-// gray(n) at and above 7 are gray(n >> 7): the CTA's paths share at most two
-// values of n >> 7, so the XOR of the upper direction numbers (with the
-// scrambler word folded in) is formed once per CTA and Sobol dimension
-// (table hi_s).  The seven low Gray bits select from two small XOR tables
-// per dimension, lo4_s (bits 0-3, 16 entries) and hi3_s (bits 4-6, 8
-// entries), so a point costs three shared-memory reads and two XORs with no
-// data-dependent branch.  Points are generated kVarBatch at a time (independent
-// work for the scheduler), then folded into the bridge, whose S points per
-// thread live in shared memory.  Output [step][factor][path] increments.
+// One thread per factor and pair of paths (p, p + 128), one CTA per factor
+// and `tiles` consecutive tiles of 256 paths.  With n = first_index + p and
+// gray(n) = n ^ (n >> 1), the bits of gray(n) at and above 7 are
+// gray(n >> 7): the first paths of a tile share at most two values h0, h0 + 1
+// of n >> 7, so the XOR of the upper direction numbers (with the scrambler
+// word folded in) is kept per CTA and Sobol dimension.  The seven low Gray
+// bits select from two small XOR tables per dimension, lo4_s (bits 0-3, 16
+// entries) and hi3_s (bits 4-6, 8 entries).  The pair's second point n + 128
+// has the same low bits of n, so it differs by Gray bit 6 and the one upper
+// bit in which gray(h + 1) differs from gray(h): one more XOR with a word
+// that is stored beside the upper XOR.  A pair of points costs three
+// shared-memory reads, with no data-dependent branch.  Points are generated
+// kVarBatch stages at a time (independent work for the scheduler), then
+// folded into the bridge, whose S points per path live in shared memory,
+// both paths of a thread in one packed FP32x2 value: the stage's weights and
+// offsets, the addressing and the loop control are read once per pair.
+// Output [step][factor][path] increments.
+//
+// Bound by the shared-memory loads and their latency (the 3.4 GB of output
+// at 2^20 paths, 80 steps and 10 factors take 0.5 ms).  Against one path per
+// thread and one tile of 128 per CTA: 1.79 -> 1.68 ms there, 138 -> 115 us at
+// 300,001 paths, 40 steps and 5 factors, 1.18 -> 1.16 ms at 200,003 paths, 120
+// steps and 15 factors (where one CTA fills an SM's shared memory).
 // ---------------------------------------------------------------------------
 constexpr int kVarBlock = 128;
+constexpr int kVarTile = 2 * kVarBlock;  // paths per tile
 constexpr int kVarBatch = 8;
+constexpr int kVarTiles = 8;  // most tiles per CTA
 
 __global__ void __launch_bounds__(kVarBlock)
-    variates_kernel(int paths, uint32_t first_index,
+    variates_kernel(int paths, uint32_t first_index, int tiles,
                     const uint32_t* __restrict__ dirs,
                     const uint32_t* __restrict__ scr, int scr_dims,
                     float* __restrict__ out,
                     const __grid_constant__ BridgePlan plan) {
   constexpr int T = kVarBlock;
+  constexpr int kRow = T * (int)sizeof(float2);  // bytes of a bridge row
   const int S = plan.steps, F = plan.factors;
   // shared memory (variates_smem_bytes): the bridge points W[S + 1][T]
   // (row S stays zero: the left neighbour of a point that has none), the
   // bridge plan per construction stage as {lw, rw, sd} weights and
   // {left row, right row, target row} byte offsets into W, and the
-  // Sobol tables hi[2][S], lo4[S][17], hi3[S][9] (rows padded by one word,
+  // Sobol tables up[2][S], lo4[S][17], hi3[S][9] (rows padded by one word,
   // so that the one-thread-per-dimension stores hit distinct banks)
-  extern __shared__ __align__(16) float W[];
+  extern __shared__ __align__(16) float var_sm[];
+  float2* W = reinterpret_cast<float2*>(var_sm);
   float4* bw_s = reinterpret_cast<float4*>(W + (size_t)(S + 1) * T);
   int4* bo_s = reinterpret_cast<int4*>(bw_s + S);
-  uint32_t* hi_s = reinterpret_cast<uint32_t*>(bo_s + S);
-  uint32_t* lo4_s = hi_s + 2 * S;
+  uint2* up_s = reinterpret_cast<uint2*>(bo_s + S);  // {upper XOR, second point's XOR}
+  uint32_t* lo4_s = reinterpret_cast<uint32_t*>(up_s + 2 * S);
   uint32_t* hi3_s = lo4_s + 17 * S;
+  const int tid = threadIdx.x;
   const int f = blockIdx.y;
   const int* alloc = plan.alloc + f * S;
-  const int p0 = blockIdx.x * kVarBlock;
-  const uint32_t h0 = (first_index + (uint32_t)p0) >> 7;
+  int p0 = blockIdx.x * tiles * kVarTile;
+  uint32_t h0 = (first_index + (uint32_t)p0) >> 7;
+  // the second points' word for upper index h: Gray bit 6 and the bit that
+  // gray(h + 1) = gray(h) ^ 2^ctz(h + 1) flips (indices below 2^31 + 256, so
+  // ctz(h + 1) <= 24 and the direction number exists)
+  auto second = [](const uint32_t* v, uint32_t h) {
+    return __ldg(v + 6) ^ __ldg(v + 7 + (__ffs(h + 1u) - 1));
+  };
   // one thread per Sobol dimension of the factor: the XOR of the direction
   // numbers over the set upper Gray bits of h0 (with the scrambler word);
-  // that of h0 + 1 differs in one Gray bit, gray(h + 1) = gray(h) ^
-  // 2^ctz(h + 1) (no entry past bit 31: h0 + 1 = 2^25 has no path); and the
-  // two low tables, each entry the previous one with its lowest set bit
-  // cleared, XOR that bit's direction number
-  for (int i = threadIdx.x; i < S; i += kVarBlock) {
+  // and the two low tables, each entry the previous one with its lowest set
+  // bit cleared, XOR that bit's direction number
+  for (int i = tid; i < S; i += T) {
     const int d = alloc[i];
     const uint32_t* v = dirs + 32 * d;
     uint32_t g = h0 ^ (h0 >> 1), x = 0;
@@ -168,12 +214,12 @@ __global__ void __launch_bounds__(kVarBlock)
       g &= g - 1u;
     }
     if (d < scr_dims) x ^= __ldg(scr + d);
-    hi_s[i] = x;
-    const int c = __ffs(h0 + 1u) - 1;
-    hi_s[S + i] = (c >= 0 && c < 25) ? x ^ __ldg(v + 7 + c) : x;
     uint32_t vl[7];
 #pragma unroll
     for (int k = 0; k < 7; ++k) vl[k] = __ldg(v + k);
+    const uint32_t d0 = second(v, h0), d1 = second(v, h0 + 1u);
+    up_s[i] = make_uint2(x, d0);
+    up_s[S + i] = make_uint2(x ^ d0 ^ vl[6], d1);
     uint32_t* l4 = lo4_s + 17 * i;
     uint32_t* h3 = hi3_s + 9 * i;
     uint32_t t4[16], t3[8];
@@ -187,73 +233,91 @@ __global__ void __launch_bounds__(kVarBlock)
     for (int e = 0; e < 16; ++e) l4[e] = t4[e];
 #pragma unroll
     for (int e = 0; e < 8; ++e) h3[e] = t3[e];
-  }
-  for (int i = threadIdx.x; i < S; i += kVarBlock) {
     // stage 0 is the terminal point W_S = sd_0 z (row S - 1); a stage
     // without a left neighbour reads the zero row S with weight 0
     const bool first = i == 0;
     const int jl = first ? 0 : plan.left[i];
     bw_s[i] = make_float4(jl != 0 ? plan.lw[i] : 0.0f, first ? 0.0f : plan.rw[i], plan.sd[i],
                           0.0f);
-    bo_s[i] = make_int4((jl != 0 ? jl - 1 : S) * T * 4, (first ? S : plan.right[i]) * T * 4,
-                        (first ? S - 1 : plan.bidx[i]) * T * 4, 0);
+    bo_s[i] = make_int4((jl != 0 ? jl - 1 : S) * kRow, (first ? S : plan.right[i]) * kRow,
+                        (first ? S - 1 : plan.bidx[i]) * kRow, 0);
   }
-  W[(size_t)S * T + threadIdx.x] = 0.0f;
+  W[(size_t)S * T + tid] = dup2(0.0f);
   __syncthreads();
-  const int p = p0 + threadIdx.x;
-  if (p >= paths) return;
-  const uint32_t n = first_index + (uint32_t)p;
-  const int sel = (int)((n >> 7) - h0);
-  const uint32_t glo = (n ^ (n >> 1)) & 127u;
-  const uint32_t ga = glo & 15u, gb = glo >> 4;
-  float* w = W + threadIdx.x;
-  // this thread's entries of the Sobol tables, stage by stage
-  const uint32_t* hi_t = hi_s + sel * S;
-  const uint32_t* lo_t = lo4_s + ga;
-  const uint32_t* h3_t = hi3_s + gb;
-  const char* wb = reinterpret_cast<const char*>(w);
-  // one batch of kVarBatch stages from i0; FULL: all of them exist (no
-  // clamp of the stage index, no guard on the bridge step)
-  auto batch = [&](int i0, auto full_tag) {
-    constexpr bool FULL = decltype(full_tag)::value;
-    float z[kVarBatch];
+  float2* w = W + tid;
+  char* wb = reinterpret_cast<char*>(w);
+  for (int t = 0; t < tiles && p0 < paths; ++t) {
+    const int p = p0 + tid;
+    const uint32_t n = first_index + (uint32_t)p;
+    const uint32_t glo = (n ^ (n >> 1)) & 127u;
+    // this thread's entries of the Sobol tables, stage by stage
+    const uint2* up_t = up_s + ((n >> 7) - h0) * S;
+    const uint32_t* lo_t = lo4_s + (glo & 15u);
+    const uint32_t* h3_t = hi3_s + (glo >> 4);
+    // one batch of kVarBatch stages from i0; FULL: all of them exist (no
+    // clamp of the stage index, no guard on the bridge step)
+    auto batch = [&](int i0, auto full_tag) {
+      constexpr bool FULL = decltype(full_tag)::value;
+      float2 z[kVarBatch];
 #pragma unroll
-    for (int k = 0; k < kVarBatch; ++k) {
-      const int i = FULL ? i0 + k : min(i0 + k, S - 1);
-      const uint32_t x = hi_t[i] ^ lo_t[17 * i] ^ h3_t[9 * i];
-      z[k] = icdf_sb_fast(x);
-    }
+      for (int k = 0; k < kVarBatch; ++k) {
+        const int i = FULL ? i0 + k : min(i0 + k, S - 1);
+        const uint2 u = up_t[i];
+        const uint32_t x = u.x ^ lo_t[17 * i] ^ h3_t[9 * i];
+        z[k] = icdf_sb_fast2(x, x ^ u.y);
+      }
 #pragma unroll
-    for (int k = 0; k < kVarBatch; ++k) {
-      const int i = i0 + k;
-      if (FULL || i < S) {
-        const float4 bw = bw_s[i];
-        const int4 bo = bo_s[i];
-        // bo: byte offsets of the stage's rows (no index scaling per access)
-        float y = bw.x * *reinterpret_cast<const float*>(wb + bo.x);
-        y = fmaf(bw.y, *reinterpret_cast<const float*>(wb + bo.y), y);
-        y = fmaf(bw.z, z[k], y);
-        *reinterpret_cast<float*>(reinterpret_cast<char*>(w) + bo.z) = y;
+      for (int k = 0; k < kVarBatch; ++k) {
+        const int i = i0 + k;
+        if (FULL || i < S) {
+          const float4 bw = bw_s[i];
+          const int4 bo = bo_s[i];
+          // bo: byte offsets of the stage's rows (no index scaling per access)
+          float2 y = __fmul2_rn(dup2(bw.x), *reinterpret_cast<const float2*>(wb + bo.x));
+          y = __ffma2_rn(dup2(bw.y), *reinterpret_cast<const float2*>(wb + bo.y), y);
+          y = __ffma2_rn(dup2(bw.z), z[k], y);
+          *reinterpret_cast<float2*>(wb + bo.z) = y;
+        }
+      }
+    };
+    if (p < paths) {
+      int i0 = 0;
+      for (; i0 + kVarBatch <= S; i0 += kVarBatch) batch(i0, std::true_type());
+      if (i0 < S) batch(i0, std::false_type());
+      float2 prev = dup2(0.0f);
+      float* o = out + (size_t)f * paths + p;
+      const size_t o_step = (size_t)F * paths;
+      const bool both = p + T < paths;
+#pragma unroll 4
+      for (int s = 0; s < S; ++s, o += o_step) {
+        const float2 cur = w[s * T];
+        o[0] = cur.x - prev.x;
+        if (both) o[T] = cur.y - prev.y;
+        prev = cur;
       }
     }
-  };
-  int i0 = 0;
-  for (; i0 + kVarBatch <= S; i0 += kVarBatch) batch(i0, std::true_type());
-  if (i0 < S) batch(i0, std::false_type());
-  float prev = 0.0f;
-  float* o = out + (size_t)f * paths + p;
-  const size_t o_step = (size_t)F * paths;
-  for (int s = 0; s < S; ++s, o += o_step) {
-    const float cur = w[s * T];
-    *o = cur - prev;
-    prev = cur;
+    p0 += kVarTile;
+    h0 += 2u;
+    if (t + 1 < tiles && p0 < paths) {  // the next tile's upper XORs
+      __syncthreads();
+      for (int i = tid; i < S; i += T) {
+        const uint32_t* v = dirs + 32 * alloc[i];
+        const uint2 last = up_s[S + i];  // of h0 - 1
+        const uint32_t v6 = __ldg(v + 6);
+        const uint32_t x = last.x ^ last.y ^ v6;
+        const uint32_t d0 = second(v, h0), d1 = second(v, h0 + 1u);
+        up_s[i] = make_uint2(x, d0);
+        up_s[S + i] = make_uint2(x ^ d0 ^ v6, d1);
+      }
+      __syncthreads();
+    }
   }
 }
 
 // Shared memory of variates_kernel for S bridge stages.
 inline size_t variates_smem_bytes(int S) {
-  return (size_t)(S + 1) * kVarBlock * sizeof(float) + (size_t)S * (sizeof(float4) + sizeof(int4)) +
-         (size_t)S * (2 + 17 + 9) * sizeof(uint32_t);
+  return (size_t)(S + 1) * kVarBlock * sizeof(float2) + (size_t)S * (sizeof(float4) + sizeof(int4)) +
+         (size_t)S * (2 * sizeof(uint2) + (17 + 9) * sizeof(uint32_t));
 }
 
 }  // namespace lmm

@@ -29,6 +29,9 @@ __device__ __forceinline__ float lg2_ftz(float x) {
 __device__ __forceinline__ float exp_ftz(float x) { return ex2_ftz(x * 1.44269504088896341f); }
 __device__ __forceinline__ float log_ftz(float x) { return lg2_ftz(x) * 0.693147180559945309f; }
 
+// Both halves of a packed FP32x2 operand.
+__device__ __forceinline__ float2 dup2(float x) { return make_float2(x, x); }
+
 // Shaw & Brickman (2009) rational approximation of the inverse cumulative
 // normal in the form used by inverseCumulativeShawBrickmanUnsignedInt
 // (inverseCumulatives.h:146-172): u = float(i) * 2^-32,
