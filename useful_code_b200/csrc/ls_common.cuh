@@ -191,18 +191,18 @@ __device__ __forceinline__ double ls_chain_estimate(const LsRuleView& r, int e, 
   return est;
 }
 
-// ls_row_estimate for two paths per thread and a known basis table: the same
+// ls_row_estimate for H paths per thread and a known basis table: the same
 // products, sums and roundings, without the generic form's exponent
 // selections (which cost about ten instructions per basis function), the
-// coefficients read once for both and two independent FP64 chains.
-template <int KIND>
-__device__ __forceinline__ void ls_row_estimate2(const double* b, const float* mean,
-                                                 const float* sd,
-                                                 const float (&v)[2][kMaxVars],
-                                                 double (&est)[2]) {
-  float pw[2][kMaxVars][3];
+// coefficients read once for all paths and H independent FP64 chains.
+template <int KIND, int H>
+__device__ __forceinline__ void ls_row_estimate_known(const double* b, const float* mean,
+                                                      const float* sd,
+                                                      const float (&v)[H][kMaxVars],
+                                                      double (&est)[H]) {
+  float pw[H][kMaxVars][3];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < H; ++h) {
     float x[kMaxVars];
 #pragma unroll
     for (int k = 0; k < kMaxVars; ++k) x[k] = mean ? (v[h][k] - mean[k]) / sd[k] : v[h][k];
@@ -213,7 +213,7 @@ __device__ __forceinline__ void ls_row_estimate2(const double* b, const float* m
   for (int k = 0; k < basis_K(KIND); ++k) {
     const double bk = b[k];
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < H; ++h)
       est[h] += (double)(ls_pow(pw[h][0], basis_exp(KIND, k, 0)) *
                          ls_pow(pw[h][1], basis_exp(KIND, k, 1)) *
                          ls_pow(pw[h][2], basis_exp(KIND, k, 2))) *
@@ -221,41 +221,51 @@ __device__ __forceinline__ void ls_row_estimate2(const double* b, const float* m
   }
 }
 
-// ls_chain_estimate for two paths per thread; kind: the date's basis kind.
-__device__ __forceinline__ void ls_chain_estimate2(const LsRuleView& r, int e, int kind,
+// ls_chain_estimate for H paths per thread; kind: the date's basis kind.
+template <int H>
+__device__ __forceinline__ void ls_chain_estimates(const LsRuleView& r, int e, int kind,
                                                    int nvars, int nbasis,
                                                    const unsigned char (*mono)[kMaxVars],
-                                                   const float (&v)[2][kMaxVars],
-                                                   const float (&exv)[2], double (&est)[2]) {
-  bool open[2] = {true, true};
-  est[0] = est[1] = 0.0;
+                                                   const float (&v)[H][kMaxVars],
+                                                   const float (&exv)[H], double (&est)[H]) {
+  bool open[H];
+#pragma unroll
+  for (int h = 0; h < H; ++h) {
+    open[h] = true;
+    est[h] = 0.0;
+  }
   for (int d = 0; d < r.depth; ++d) {
     const size_t row = (size_t)e * r.depth + d;
     const double* b = r.beta + row * kMaxBasis;
     const float* mean = r.means ? r.means + row * kMaxVars : nullptr;
     const float* sd = r.means ? r.sds + row * kMaxVars : nullptr;
-    double t[2];
+    double t[H];
     switch (kind) {
-      case kBasisC2: ls_row_estimate2<kBasisC2>(b, mean, sd, v, t); break;
-      case kBasisQuad: ls_row_estimate2<kBasisQuad>(b, mean, sd, v, t); break;
-      case kBasisCross: ls_row_estimate2<kBasisCross>(b, mean, sd, v, t); break;
-      case kBasisC5: ls_row_estimate2<kBasisC5>(b, mean, sd, v, t); break;
+      case kBasisC2: ls_row_estimate_known<kBasisC2>(b, mean, sd, v, t); break;
+      case kBasisQuad: ls_row_estimate_known<kBasisQuad>(b, mean, sd, v, t); break;
+      case kBasisCross: ls_row_estimate_known<kBasisCross>(b, mean, sd, v, t); break;
+      case kBasisC5: ls_row_estimate_known<kBasisC5>(b, mean, sd, v, t); break;
       default:
 #pragma unroll 1
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < H; ++h) {
           float x[kMaxVars];
 #pragma unroll
-          for (int k = 0; k < kMaxVars; ++k) x[k] = h ? v[1][k] : v[0][k];
+          for (int k = 0; k < kMaxVars; ++k) {
+            x[k] = v[0][k];
+#pragma unroll
+            for (int g = 1; g < H; ++g)
+              if (h == g) x[k] = v[g][k];
+          }
           const double y = ls_row_estimate(b, mean, sd, nvars, nbasis, mono, x);
-          if (h)
-            t[1] = y;
-          else
-            t[0] = y;
+#pragma unroll
+          for (int g = 0; g < H; ++g)
+            if (h == g) t[g] = y;
         }
     }
     const double shift = r.shifts ? (double)r.shifts[e] : 0.0;
+    bool any = false;
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+    for (int h = 0; h < H; ++h) {
       if (open[h]) {
         est[h] = shift + t[h];
         if (d + 1 < r.depth && r.cuts) {
@@ -263,7 +273,9 @@ __device__ __forceinline__ void ls_chain_estimate2(const LsRuleView& r, int e, i
           open[h] = net > r.cuts[row * 2] && net < r.cuts[row * 2 + 1];
         }
       }
-    if (!r.cuts || !(open[0] || open[1])) break;
+      any = any || open[h];
+    }
+    if (!r.cuts || !any) break;
   }
 }
 #endif

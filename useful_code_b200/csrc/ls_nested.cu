@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kNestThreads)
                          : 1.0f;
     }
     double est[2];
-    ls_chain_estimate2(rule, e, kind, dd.nvars, dd.nbasis, dd.mono, v, exv, est);
+    ls_chain_estimates<2>(rule, e, kind, dd.nvars, dd.nbasis, dd.mono, v, exv, est);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (h && !two) break;
@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(kSelThreads, 1)
       exv[h] = ex ? ex[(size_t)e * paths + p[h]] : 0.0f;
     }
     double est[2];
-    ls_chain_estimate2(one, 0, a.kind, a.dd.nvars, a.dd.nbasis, a.dd.mono, v, exv, est);
+    ls_chain_estimates<2>(one, 0, a.kind, a.dd.nvars, a.dd.nbasis, a.dd.mono, v, exv, est);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (h && !two) break;

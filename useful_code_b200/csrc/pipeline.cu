@@ -162,6 +162,7 @@ int validate(const lmm_model* m, const lmm_product* pr, Validated* v) {
       if (st) return st;
       v->rc.nvars[e] = d.nvars;
       v->rc.nbasis[e] = d.nbasis;
+      v->rc.kind[e] = (unsigned char)ls_basis_kind(d);
       memcpy(v->rc.mono[e], d.mono, sizeof(d.mono));
     }
   }
@@ -411,12 +412,13 @@ int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
                  RecordOut rec = RecordOut{nullptr, nullptr, nullptr, 1},
                  const SegIO* segment = nullptr) {
   const int block = kFusedBlock;
-  const size_t smem = fused_smem_bytes(v.n, v.F, block);
   const int grid = div_up(P, block);
   SegIO whole{};
   whole.s_begin = 0;
   whole.s_end = v.n;
   const SegIO& sg = segment ? *segment : whole;
+  // only the rates alive at the launch's first step have rows
+  const size_t smem = fused_smem_bytes(v.n - sg.s_begin, v.F, block);
   auto go = [&](auto kern) -> int {
     TRY(check_cuda(cudaFuncSetAttribute(kern,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1029,7 +1031,7 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
   const double P0 = 1.0 / (1.0 + (double)model->h_initial_rates[0] * (double)t0);
   const double scale = P0 / (double)P;
   const int block_seg = kRevThreads;  // one tile of the reverse sweep per CTA
-  const size_t smem_seg = fused_smem_bytes(n, F, block_seg);
+  const size_t smem_seg = segment_smem_bytes(n, F, block_seg);
   const size_t smem_rev = greeks_reverse_smem(n, F);
   // persistent CTAs: as many as are resident at once (at most the bound)
   int grid_rev = greeks_reverse_grid(P);
