@@ -394,12 +394,15 @@ __device__ __forceinline__ void stage_rows(float* As, float* fx, const float* __
 // Fused evolution.  One thread per path, CTA of 128 paths; shared memory
 // holds the CTA's log-rates [rate][thread] and the alive rows of the step's
 // pseudo-root (padded to a multiple of 4 factors for 16-byte loads) and
-// fixed drift.  A step must not wait for memory: its rows are copied one step ahead into the other of two buffers
+// fixed drift.  Launches too small for two paths per thread (fused_pairs.cuh)
+// run it, with a few warps per SM or fewer, so a step must not wait for
+// memory: its rows are copied one step ahead into the other of two buffers
 // (cp.async; one barrier per step) and its normals loaded one step ahead.
 // With both and the exercise rule's known tables (launches bound by latency):
 // 20 rates, 3 factors, 16,384 paths 52 -> 46 us with the variates; 80 rates,
 // 10 factors, 16,384 paths 0.470 -> 0.366 ms, the frozen-rule chain 0.80 ->
-// 0.60 ms; 120 rates, 15 factors, 10,000 paths, the chain 1.72 -> 1.23 ms.  Per rate and step: predictor drift from the rates at the start of
+// 0.60 ms; 120 rates, 15 factors, 10,000 paths, the chain 1.72 -> 1.23 ms.
+// Per rate and step: predictor drift from the rates at the start of
 // the step, predicted log-rate, corrector drift, corrected and capped
 // log-rate (LMM_evolver_all.cu:615-744, gold/LMM_evolver_gold.h:315-387);
 // the spot drift factor is g = F tau / (1 + f tau) with F = f + d the

@@ -113,4 +113,178 @@ __device__ __forceinline__ void step_start(const float (&z)[FP], float2 (&w)[FP 
   }
 }
 
+// pc_rate for two paths per thread: the pair's values in the two halves of a
+// float2 and the factor vectors w, v as one float2 per factor, so that every
+// operation of the rate step (not only the factor sums) is one packed
+// instruction for both paths and the pseudo-root row, the constants and the
+// loop control are read once per pair.  Each half runs pc_rate's own sequence
+// of roundings (even and odd factors in two accumulators, added last), so a
+// path's values are bit-identical to pc_rate's.
+__device__ __forceinline__ float2 cap2(float2 lf, float cutoff) {
+  return make_float2(fminf(lf.x, cutoff), fminf(lf.y, cutoff));
+}
+
+template <int FM, int FP>
+__device__ __forceinline__ float2 pc_rate2(float2 lf, float l2tau, float c0, float fxr,
+                                           const float* Arow, float2 (&w)[FM], float2 (&v)[FM],
+                                           float2& g, float2& gp, float2& q) {
+  constexpr float kLog2e = 1.44269504088896341f;
+  const float4* a4 = reinterpret_cast<const float4*>(Arow);
+  float a[FP];
+#pragma unroll
+  for (int k = 0; k < FP / 4; ++k) {
+    const float4 t = a4[k];
+    a[4 * k] = t.x;
+    a[4 * k + 1] = t.y;
+    a[4 * k + 2] = t.z;
+    a[4 * k + 3] = t.w;
+  }
+  float2 dw[2] = {dup2(0.0f), dup2(0.0f)}, dv[2] = {dup2(0.0f), dup2(0.0f)};
+#pragma unroll
+  for (int f = 0; f < FM; ++f) {
+    dw[f & 1] = __ffma2_rn(dup2(a[f]), w[f], dw[f & 1]);
+    dv[f & 1] = __ffma2_rn(dup2(a[f]), v[f], dv[f & 1]);
+  }
+  const float2 nA2 = dup2(-2.0f * fxr);
+  float2 t = __ffma2_rn(lf, dup2(kLog2e), dup2(l2tau));
+  const float2 Fr = make_float2(ex2_ftz(t.x), ex2_ftz(t.y));
+  t = __fadd2_rn(dup2(c0), Fr);
+  q = make_float2(rcp_ftz(t.x), rcp_ftz(t.y));
+  g = __fmul2_rn(Fr, q);
+  lf = __fadd2_rn(lf, __fadd2_rn(__ffma2_rn(g, nA2, __fadd2_rn(dw[0], dw[1])), dup2(fxr)));
+  t = __ffma2_rn(lf, dup2(kLog2e), dup2(l2tau));
+  const float2 Fp = make_float2(ex2_ftz(t.x), ex2_ftz(t.y));
+  t = __fadd2_rn(dup2(c0), Fp);
+  const float2 qp = make_float2(rcp_ftz(t.x), rcp_ftz(t.y));
+  gp = __fmul2_rn(Fp, qp);
+  const float2 dg = __ffma2_rn(Fp, qp, make_float2(-g.x, -g.y));
+  lf = __ffma2_rn(dup2(0.5f), __ffma2_rn(dg, nA2, __fadd2_rn(dv[0], dv[1])), lf);
+#pragma unroll
+  for (int f = 0; f < FM; ++f) {
+    w[f] = __ffma2_rn(dup2(a[f]), g, w[f]);
+    v[f] = __ffma2_rn(dup2(a[f]), dg, v[f]);
+  }
+  return lf;
+}
+
+// Tensor memory as storage: allocation of `cols` columns (a power of two) by
+// one warp, eight columns of the calling warp's lanes at a time.
+__host__ __device__ __forceinline__ uint32_t tmem_columns(int rows) {
+  uint32_t c = rows > 0 ? 32u : 0u;
+  while (c < 2u * (uint32_t)rows) c *= 2u;
+  return c;
+}
+// `cols` may be 0.  The CTA gives up its right to allocate in either case:
+// until a CTA of a kernel with tensor-memory instructions has done so, its SM
+// starts no further CTA of the kernel (1 instead of 4 CTAs per SM measured
+// without it, 0.92 against 0.44 ms for 2^18 paths of 40 rates).
+__device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
+  if (cols)
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(slot)),
+                 "r"(cols)
+                 : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_fence_before() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_fence_after() {
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t a, const float2 (&x)[4]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(a),
+      "f"(x[0].x), "f"(x[0].y), "f"(x[1].x), "f"(x[1].y), "f"(x[2].x), "f"(x[2].y),
+      "f"(x[3].x), "f"(x[3].y)
+      : "memory");
+}
+// waits for this thread's earlier stores, loads, and waits for the load
+__device__ __forceinline__ void tmem_ld8(uint32_t a, float2 (&x)[4]) {
+  asm volatile(
+      "tcgen05.wait::st.sync.aligned;\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=f"(x[0].x), "=f"(x[0].y), "=f"(x[1].x), "=f"(x[1].y), "=f"(x[2].x), "=f"(x[2].y),
+        "=f"(x[3].x), "=f"(x[3].y)
+      : "r"(a)
+      : "memory");
+}
+
+// A thread's log-rates of its two paths: rates s_begin .. nt0 - 1 in shared
+// memory, row r at row[(r - s_begin) * T]; rates nt0 .. n - 1 (a multiple of
+// four of them) in tensor memory, two columns each from column `tmem` of the
+// warp's lanes.
+template <int T>
+struct LogRates {
+  float2* row;
+  uint32_t tmem;
+  int s_begin, nt0;
+  // fn(r, pair) for the rates r = s .. n - 1 (whole warps)
+  template <class Fn>
+  __device__ __forceinline__ void for_each(int s, int n, Fn&& fn) const {
+    for (int r = s; r < nt0; ++r) fn(r, row[(r - s_begin) * T]);
+    for (int r0 = nt0 + (max(s - nt0, 0) & ~3); r0 < n; r0 += 4) {
+      float2 x[4];
+      tmem_ld8(tmem + 2 * (r0 - nt0), x);
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (r0 + j >= s) fn(r0 + j, x[j]);
+    }
+  }
+};
+
+// One step: pc_rate2 over the rates s .. n - 1 of the log-rates lr (whole
+// warps).  As, fx: the step's rows, rate r at row r - s.  hook(r, g, gp, q,
+// ln): called per rate with pc_rate2's outputs and the new log-rates before
+// the cap.  Returns the new log-rates of rate s.
+template <int FM, int FP, int T, class Hook>
+__device__ __forceinline__ float2 pc_step2(const LogRates<T>& lr, int s, int n,
+                                           const ModelConst& mc, const float* As,
+                                           const float* fx, float2 (&w)[FM], float2 (&v)[FM],
+                                           Hook&& hook) {
+  auto rate = [&](int r, float2 lf) {
+    float2 g, gp, q;
+    const int i = r - s;
+    lf = pc_rate2<FM, FP>(lf, mc.l2tau[r], mc.c0[r], fx[i], As + i * FP, w, v, g, gp, q);
+    hook(r, g, gp, q, lf);
+    return cap2(lf, mc.cutoff);
+  };
+  float2 lf0 = dup2(0.0f);
+  float2* row = lr.row + (s - lr.s_begin) * T;
+#pragma unroll 4
+  for (int r = s; r < lr.nt0; ++r) row[(r - s) * T] = rate(r, row[(r - s) * T]);
+  int r0 = lr.nt0;
+  if (s < lr.nt0) {
+    lf0 = row[0];
+  } else {  // the step starts inside the tensor-memory rows, maybe inside a block
+    r0 += (s - lr.nt0) & ~3;
+    float2 x[4];
+    const uint32_t a = lr.tmem + 2 * (r0 - lr.nt0);
+    tmem_ld8(a, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (r0 + j >= s) {
+        x[j] = rate(r0 + j, x[j]);
+        if (r0 + j == s) lf0 = x[j];
+      }
+    tmem_st8(a, x);
+    r0 += 4;
+  }
+#pragma unroll 1
+  for (; r0 < n; r0 += 4) {
+    float2 x[4];
+    const uint32_t a = lr.tmem + 2 * (r0 - lr.nt0);
+    tmem_ld8(a, x);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j] = rate(r0 + j, x[j]);
+    tmem_st8(a, x);
+  }
+  return lf0;
+}
+
 }  // namespace lmm

@@ -26,6 +26,7 @@
 #include "ls_common.cuh"
 #include "../../include/lmm_pipeline.h"
 #include "fused_kernels.cuh"
+#include "fused_pairs.cuh"
 #include "greeks_kernels.cuh"
 #include "tc_evolve.cuh"
 #include "ab_kernels.cuh"
@@ -404,6 +405,39 @@ int staged_cap_add(const lmm_model* m, const lmm_product* pr, const Validated& v
   return check_launch("sum3_kernel");
 }
 
+// Calls go(std::integral_constant<int, FT>) with the compiled factor count
+// (0 = generic).
+template <class Fn>
+int dispatch_factors(int F, Fn&& go) {
+  switch (F) {
+    case 3: return go(std::integral_constant<int, 3>());
+    case 5: return go(std::integral_constant<int, 5>());
+    case 10: return go(std::integral_constant<int, 10>());
+    case 15: return go(std::integral_constant<int, 15>());
+    default: return go(std::integral_constant<int, 0>());
+  }
+}
+
+// Two paths per thread (fused_pairs.cuh) where the pairs still fill the GPU,
+// else one: with fewer paths the halved number of warps costs more than the
+// pairs save.  Measured (one against two paths per thread): one launch of 80
+// rates and 10 factors 0.60 / 0.67 ms at 50,000 paths, 0.76 / 0.67 at 65,536,
+// 1.44 / 1.22 at 150,000; of 120 rates and 15 factors 1.20 / 1.11 at 20,480,
+// 2.37 / 1.80 at 65,536; of 40 rates and 5 factors 0.129 / 0.145 at 37,000,
+// 0.181 / 0.175 at 65,536, 0.55 / 0.44 at 2^18.  In a chain of segments the
+// later launches hold few survivors: 80 rates 0.87 / 0.95 at 65,536, 1.21 /
+// 1.15 at 110,000; 120 rates 1.83 / 2.05 at 65,536; 40 rates 0.32 / 0.35 at
+// 110,000.  Few rates and factors (20 and 3: 57 / 62 us at 65,536) leave a
+// step too little arithmetic to pair.
+bool use_pairs(const Validated& v, int P, bool chain) {
+  if ((long long)P * v.n * v.F < (1ll << 23)) return false;
+  if (chain) return P >= (v.F >= 10 ? 100000 : 160000);
+  return P >= (v.F > 10 ? 20480 : 56000);
+}
+int evolve_block(const Validated& v, int P, bool chain) {
+  return use_pairs(v, P, chain) ? kPairBlock : kFusedBlock;
+}
+
 template <int MODE>
 int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
                  const LsRuleView& rule,
@@ -411,31 +445,37 @@ int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
                  float* num, float* payoff, cudaStream_t s,
                  RecordOut rec = RecordOut{nullptr, nullptr, nullptr, 1},
                  const SegIO* segment = nullptr) {
-  const int block = kFusedBlock;
+  const bool pairs = use_pairs(v, P, segment != nullptr);
+  const int block = pairs ? kPairBlock : kFusedBlock;
   const int grid = div_up(P, block);
   SegIO whole{};
   whole.s_begin = 0;
   whole.s_end = v.n;
   const SegIO& sg = segment ? *segment : whole;
-  // only the rates alive at the launch's first step have rows
-  const size_t smem = fused_smem_bytes(v.n - sg.s_begin, v.F, block);
-  auto go = [&](auto kern) -> int {
-    TRY(check_cuda(cudaFuncSetAttribute(kern,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem),
-                   "fused: smem attribute"));
-    kern<<<grid, block, smem, s>>>(P, Z, m->d_A, m->d_fixed_drifts, v.mc, v.pc,
-                                   v.rc, rule, total, col, vars, ex,
-                                   cf, num, payoff, rec, sg);
-    return check_launch("fused_evolve_kernel");
+  const int rows = v.n - sg.s_begin;  // rates alive at the launch's first step
+  const int tmem_rows = pairs ? pair_tmem_rows(rows, v.F) : 0;
+  const size_t smem = pairs ? pair_smem_bytes(rows, v.F, rows - tmem_rows)
+                                   : fused_smem_bytes(rows, v.F, block);
+  auto attr = [&](auto kern) -> int {
+    return check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem),
+                      "fused: smem attribute");
   };
-  switch (v.F) {
-    case 3: return go(fused_evolve_kernel<3, MODE>);
-    case 5: return go(fused_evolve_kernel<5, MODE>);
-    case 10: return go(fused_evolve_kernel<10, MODE>);
-    case 15: return go(fused_evolve_kernel<15, MODE>);
-    default: return go(fused_evolve_kernel<0, MODE>);
-  }
+  return dispatch_factors(v.F, [&](auto ft) -> int {
+    constexpr int FT = decltype(ft)::value;
+    if (pairs) {
+      TRY(attr(fused_pairs_kernel<FT, MODE>));
+      fused_pairs_kernel<FT, MODE><<<grid, kPairThreads, smem, s>>>(
+          P, Z, m->d_A, m->d_fixed_drifts, v.mc, v.pc, v.rc, rule, total, col, vars, ex, cf, num,
+          payoff, rec, sg, v.n - tmem_rows);
+      return check_launch("fused_pairs_kernel");
+    }
+    TRY(attr(fused_evolve_kernel<FT, MODE>));
+    fused_evolve_kernel<FT, MODE><<<grid, block, smem, s>>>(
+        P, Z, m->d_A, m->d_fixed_drifts, v.mc, v.pc, v.rc, rule, total, col, vars, ex, cf, num,
+        payoff, rec, sg);
+    return check_launch("fused_evolve_kernel");
+  });
 }
 
 // Segmented rule-mode second pass (SegIO, fused_kernels.cuh): products whose
@@ -458,8 +498,9 @@ struct SegBufs {
 
 SegBufs carve_seg(Carver& c, const Validated& v, int P) {
   SegBufs b;
-  b.blocks = div_up(P, kFusedBlock);
-  b.cap = b.blocks * kFusedBlock;
+  const int block = evolve_block(v, P, true);
+  b.blocks = div_up(P, block);
+  b.cap = b.blocks * block;
   const size_t cap = (size_t)b.cap;
   for (SegState& st : b.st) {
     st.rates = c.take<float>((size_t)v.n * cap);
@@ -603,18 +644,6 @@ GreeksBufs carve_greeks(Carver& c, const Validated& v, size_t P, int k) {
   return b;
 }
 
-// Calls go(std::integral_constant<int, FT>) with the compiled factor count
-// (0 = generic).
-template <class Fn>
-int dispatch_factors(int F, Fn&& go) {
-  switch (F) {
-    case 3: return go(std::integral_constant<int, 3>());
-    case 5: return go(std::integral_constant<int, 5>());
-    case 10: return go(std::integral_constant<int, 10>());
-    case 15: return go(std::integral_constant<int, 15>());
-    default: return go(std::integral_constant<int, 0>());
-  }
-}
 
 size_t workspace_bytes(const Validated& v, int paths, int mode) {
   Carver c{nullptr};
