@@ -1369,23 +1369,18 @@ extern "C" int lmm_andersen_broadie(const lmm_model* model, const lmm_product* p
   a.k1 = (uint32_t)(cfg->seed >> 32);
   for (int s2 = 0, e = 0; s2 < n; ++s2)
     if (v.pc.ex_index[s2] >= 0) a.ex_step[e++] = s2;
-  const size_t smem = ab_inner_smem(n);
-  const unsigned grid = (unsigned)((size_t)(E - 1) * K * chunks);
-  auto go = [&](auto kern) -> int {
+  const int tmem_rows = pair_tmem_rows(n, v.F);
+  const size_t smem = pair_smem_bytes(n, v.F, n - tmem_rows);
+  const unsigned grid = (unsigned)((size_t)(E - 1) * (((size_t)K * chunks + 1) / 2));
+  TRY(dispatch_factors(v.F, [&](auto ft) -> int {
+    auto kern = ab_inner_kernel<decltype(ft)::value>;
     TRY(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem),
                    "ab_inner: smem attribute"));
-    kern<<<grid, kAbThreads, smem, s>>>(a, model->d_A, model->d_fixed_drifts, v.mc, v.pc, v.rc,
-                                        view, b.ckpt, b.ckptN, b.part);
+    kern<<<grid, kPairThreads, smem, s>>>(a, model->d_A, model->d_fixed_drifts, v.mc, v.pc, v.rc,
+                                          view, b.ckpt, b.ckptN, b.part, n - tmem_rows);
     return check_launch("ab_inner_kernel");
-  };
-  switch (v.F) {
-    case 3: TRY(go(ab_inner_kernel<3>)); break;
-    case 5: TRY(go(ab_inner_kernel<5>)); break;
-    case 10: TRY(go(ab_inner_kernel<10>)); break;
-    case 15: TRY(go(ab_inner_kernel<15>)); break;
-    default: TRY(go(ab_inner_kernel<0>)); break;
-  }
+  }));
   ab_continuation_kernel<<<div_up(E * K, 256), 256, 0, s>>>(E, K, chunks, cfg->inner_paths,
                                                            b.part, b.Q, nullptr);
   TRY(check_launch("ab_continuation_kernel"));
