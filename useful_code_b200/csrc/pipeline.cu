@@ -594,12 +594,12 @@ struct GreeksBufs {
   float *seg[2], *seg_info[2];
   int* ex_step;
   double *later, *lam_sum, *mean, *red;
-  // the reverse launches' per-CTA partials, step s in part[s & 1]: a launch
-  // sums the previous one's while writing its own
+  // the reverse launches' per-CTA partials, alternating: a launch sums the
+  // previous one's while writing its own
   double* part[2];
   // the paths' order for the reverse sweep, and a segment's checkpoint and
   // normals in it (the normals, read by the reverse sweep too, twice)
-  int *perm, *ex_sorted, *cnt, *live, *tile_list;
+  int *perm, *ex_sorted, *cnt;
   float *ckS, *ckNS, *Zs[2];
 };
 
@@ -628,7 +628,8 @@ GreeksBufs carve_greeks(Carver& c, const Validated& v, size_t P, int k) {
   b.lam = c.take<float>(n * P);
   b.later = c.take<double>(P);
   for (int i = 0; i < 2; ++i)
-    b.part[i] = c.take<double>((size_t)greeks_reverse_grid((int)P) * greeks_part_width(n, F));
+    b.part[i] = c.take<double>((size_t)std::min(k, kRevSteps) * greeks_reverse_grid((int)P) *
+                               greeks_part_width(n, F));
   b.lam_sum = c.take<double>(n);
   b.mean = c.take<double>(1);
   b.red = c.take<double>(512);
@@ -636,8 +637,6 @@ GreeksBufs carve_greeks(Carver& c, const Validated& v, size_t P, int k) {
   b.perm = c.take<int>(P);
   b.ex_sorted = c.take<int>(P);
   b.cnt = c.take<int>(n * chunks);
-  b.live = c.take<int>(n);
-  b.tile_list = c.take<int>(n * ((P + kRevThreads - 1) / kRevThreads));
   b.ckS = c.take<float>(n * P);
   b.ckNS = c.take<float>(P);
   for (int i = 0; i < 2; ++i) b.Zs[i] = c.take<float>((size_t)k * F * P);
@@ -1059,24 +1058,47 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
                  "lmm_greeks: clear flows"));
   const double P0 = 1.0 / (1.0 + (double)model->h_initial_rates[0] * (double)t0);
   const double scale = P0 / (double)P;
-  const int block_seg = kRevThreads;  // one tile of the reverse sweep per CTA
-  const size_t smem_seg = segment_smem_bytes(n, F, block_seg);
+  // the recompute: one tile of the reverse sweep per CTA, or two with pairs
+  const bool pairs = use_pairs(v, P, false);
+  const int block_seg = pairs ? kPairBlock : kRevThreads;
+  auto seg_smem = [&](int s0) {
+    return pairs ? pair_smem_bytes(n - s0, F, n - s0 - pair_tmem_rows(n - s0, F))
+                 : segment_smem_bytes(n, F, block_seg);
+  };
+  size_t smem_seg = 0;
+  for (int s0 = 0; s0 < n; s0 += k) smem_seg = std::max(smem_seg, seg_smem(s0));
   const size_t smem_rev = greeks_reverse_smem(n, F);
-  // persistent CTAs: as many as are resident at once (at most the bound)
+  // persistent CTAs: as many as are resident at once (at most the bound), with
+  // one path per thread when all tiles are
   int grid_rev = greeks_reverse_grid(P);
-  TRY(dispatch_factors(F, [&](auto ft) -> int {
-    constexpr int FT = decltype(ft)::value;
-    auto kern = greeks_reverse_kernel<FT>;
-    TRY(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem_rev),
-                   "greeks: reverse smem"));
-    int per_sm = 0;
-    TRY(check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRevThreads,
-                                                                 smem_rev),
-                   "greeks: occupancy"));
-    grid_rev = std::max(1, std::min(grid_rev, std::max(per_sm, 1) * sm_count()));
-    return LMM_OK;
-  }));
+  bool rev_one = false;
+  auto dispatch_reverse = [&](auto&& go) -> int {
+    return dispatch_factors(F, [&](auto ft) -> int {
+      constexpr int FT = decltype(ft)::value;
+      return rev_one ? go(greeks_reverse_kernel<FT, 1>) : go(greeks_reverse_kernel<FT, 2>);
+    });
+  };
+  auto resident = [&](int* ctas) -> int {
+    return dispatch_reverse([&](auto kern) -> int {
+      TRY(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                          (int)smem_rev),
+                     "greeks: reverse smem"));
+      int per_sm = 0;
+      TRY(check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRevThreads,
+                                                                   smem_rev),
+                     "greeks: occupancy"));
+      *ctas = std::max(per_sm, 1) * sm_count();
+      return LMM_OK;
+    });
+  };
+  int ctas = 0;
+  rev_one = true;
+  TRY(resident(&ctas));
+  if (div_up(P, kRevThreads) > ctas) {
+    rev_one = false;
+    TRY(resident(&ctas));
+  }
+  grid_rev = std::max(1, std::min(grid_rev, ctas));
   const int abar_entries = n * F + n;  // dV/dA_s and the adjoint sums
   const int C = (n + k - 1) / k;
   const int stop_rule = product->kind == LMM_PRODUCT_SWAPTION ? 1
@@ -1090,9 +1112,6 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
     greeks_sort_kernel<<<chunks, kSortThreads, 0, s>>>(P, n, stop_rule, b.ex_step, chunks,
                                                         b.perm, b.ex_sorted, b.cnt);
     TRY(check_launch("greeks_sort_kernel"));
-    greeks_live_tiles_kernel<<<n, 32, 0, s>>>(chunks, div_up(P, kRevThreads), b.cnt, b.live,
-                                              b.tile_list);
-    TRY(check_launch("greeks_live_tiles_kernel"));
   }
   const int* ex_rev = ordered ? b.ex_sorted : b.ex_step;
   const int* cnt = ordered ? b.cnt : nullptr;
@@ -1105,8 +1124,9 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
   TRY(greeks_streams(&gs));
   TRY(dispatch_factors(F, [&](auto ft) -> int {
     constexpr int FT = decltype(ft)::value;
-    return check_cuda(cudaFuncSetAttribute(greeks_segment_kernel<FT>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const void* kern = pairs ? (const void*)greeks_segment_pairs_kernel<FT>
+                             : (const void*)greeks_segment_kernel<FT>;
+    return check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem_seg),
                       "greeks: segment smem");
   }));
@@ -1135,35 +1155,45 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
     }
     TRY(dispatch_factors(F, [&](auto ft) -> int {
       constexpr int FT = decltype(ft)::value;
-      greeks_segment_kernel<FT><<<div_up(P, block_seg), block_seg, smem_seg, gs->lo>>>(
-          P, s0, s1, Zseg, zs0, cnt, chunks, model->d_A, model->d_fixed_drifts, v.mc, ck, ckN,
-          ex_rev, stop_rule, b.seg[bi], b.seg_info[bi]);
+      if (pairs)
+        greeks_segment_pairs_kernel<FT>
+            <<<div_up(P, block_seg), kPairThreads, seg_smem(s0), gs->lo>>>(
+                P, s0, s1, n - pair_tmem_rows(n - s0, F), Zseg, zs0, cnt, chunks, model->d_A,
+                model->d_fixed_drifts, v.mc, ck, ckN, ex_rev, stop_rule, b.seg[bi],
+                b.seg_info[bi]);
+      else
+        greeks_segment_kernel<FT><<<div_up(P, block_seg), block_seg, seg_smem(s0), gs->lo>>>(
+            P, s0, s1, Zseg, zs0, cnt, chunks, model->d_A, model->d_fixed_drifts, v.mc, ck, ckN,
+            ex_rev, stop_rule, b.seg[bi], b.seg_info[bi]);
       return check_launch("greeks_segment_kernel");
     }));
     return check_cuda(cudaEventRecord(gs->seg_done[bi], gs->lo), "lmm_greeks: event");
   };
+  int rev_launch = 0, prev_hi = 0, prev_steps = 0;
   auto sweep = [&](int cp) -> int {  // on gs->hi
     int s0, s1;
     seg_range(cp, s0, s1);
     const int bi = cp & 1;
-    const float* Zseg = ordered ? b.Zs[bi] : b.Z;
-    const int zs0 = ordered ? s0 : 0;
     TRY(check_cuda(cudaStreamWaitEvent(gs->hi, gs->seg_done[bi], 0), "lmm_greeks: wait"));
-    for (int st = s1 - 1; st >= s0; --st) {
-      // this launch writes step st's partials and first sums step st + 1's
-      GreeksStepBufs gb{b.lam, b.later, b.part[st & 1]};
-      const GreeksPrevSums prev{st + 1 < n ? b.part[(st + 1) & 1] : nullptr, st + 1, grid_rev,
-                                scale, d_abar};
-      const size_t ko = (size_t)(st - s0);
-      GreeksStepIn in{b.seg[bi] + ko * (greeks_seg_floats(n, P, 1)),
-                      b.seg_info[bi] + ko * (2 * F + 3) * P};
-      TRY(dispatch_factors(F, [&](auto ft) -> int {
-        constexpr int FT = decltype(ft)::value;
-        greeks_reverse_kernel<FT><<<grid_rev, kRevThreads, smem_rev, gs->hi>>>(
-            P, st, Zseg, zs0, ordered ? b.live : nullptr, ordered ? b.tile_list : nullptr,
-            model->d_A, v.mc, v.pc, in, ex_rev, gb, prev);
+    for (int hi = s1 - 1; hi >= s0; hi -= kRevSteps) {
+      // this launch writes its steps' partials and first sums the launch
+      // before's
+      const int lo = std::max(s0, hi - kRevSteps + 1);
+      GreeksStepBufs gb{b.lam, b.later, b.part[rev_launch & 1]};
+      const GreeksPrevSums prev{rev_launch ? b.part[(rev_launch - 1) & 1] : nullptr,
+                                prev_hi, prev_steps, grid_rev, scale, d_abar};
+      const size_t ko = (size_t)(hi - s0);
+      const size_t seg_stride = greeks_seg_floats(n, P, 1), info_stride = (size_t)(2 * F + 3) * P;
+      GreeksStepIn in{b.seg[bi] + ko * seg_stride, b.seg_info[bi] + ko * info_stride, seg_stride,
+                      info_stride};
+      TRY(dispatch_reverse([&](auto kern) -> int {
+        kern<<<grid_rev, kRevThreads, smem_rev, gs->hi>>>(P, hi, lo, cnt, chunks, model->d_A,
+                                                          v.mc, v.pc, in, ex_rev, gb, prev);
         return check_launch("greeks_reverse_kernel");
       }));
+      prev_hi = hi;
+      prev_steps = hi - lo + 1;
+      ++rev_launch;
     }
     return check_cuda(cudaEventRecord(gs->rev_done[bi], gs->hi), "lmm_greeks: event");
   };
@@ -1181,11 +1211,12 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
         TRY(recompute(cp - 2));
       }
     }
-    // step 0's dV/dA and the rate adjoints behind the deltas (the other
-    // steps' sums ran at the start of the next reverse launch)
-    greeks_abar_kernel<<<div_up((long long)abar_entries * 32, kAbarThreads), kAbarThreads, 0,
-                         gs->hi>>>(n, F, 0, grid_rev, scale, b.part[0], model->d_A, d_abar,
-                                   b.lam_sum);
+    // the last launch's dV/dA and the rate adjoints behind the deltas (the
+    // other launches' sums ran at the start of the next one)
+    greeks_abar_kernel<<<div_up((long long)abar_entries * prev_steps * 32, kAbarThreads),
+                         kAbarThreads, 0, gs->hi>>>(n, F, prev_hi, prev_steps, grid_rev, scale,
+                                                    b.part[(rev_launch - 1) & 1], model->d_A,
+                                                    d_abar, b.lam_sum);
     return check_launch("greeks_abar_kernel");
   }();
   // join both streams (after a failed launch too, so that nothing the call
