@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
       __threadfence();
       atomicAdd(counter, 1u);
       int ok = 0;
-      for (int i = 0; i < (1 << 22) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
+      for (int i = 0; i < (1 << 25) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
       __threadfence();
       ok_s = ok;
     }
@@ -965,6 +965,7 @@ __global__ void ls_moments_final_kernel(const double* __restrict__ part,
   if (i >= n_ex * kMaxVars) return;
   const int e = i / kMaxVars, v = i % kMaxVars;
   double s = 0.0, s2 = 0.0;
+#pragma unroll 8
   for (int b = 0; b < nblocks; ++b) {
     s += part[((size_t)e * nblocks + b) * 6 + 2 * v];
     s2 += part[((size_t)e * nblocks + b) * 6 + 2 * v + 1];
@@ -1002,11 +1003,16 @@ int ls_fill_date(const LSBasisSpec& spec, int e, LSDate* d) {
 // One CTA per SM for the date kernels and the moments.
 int ls_gram_blocks() { return sm_count(); }
 
+// CTAs per date of the moments: four paths per thread or more.
+static int moment_blocks(int paths) {
+  return std::min(ls_gram_blocks(), div_up(paths, 1024));
+}
+
 // Moments of every date's basis variables over all paths into row e * rows
 // of means / sds; part: n_ex * ls_gram_blocks() * 6 doubles.
 int ls_moments_launch(const float* vars, int paths, int n_ex, int rows, float* means,
                       float* sds, double* part, cudaStream_t s) {
-  const int nblk = ls_gram_blocks();
+  const int nblk = moment_blocks(paths);
   ls_moments_kernel<<<dim3(nblk, n_ex), 256, 0, s>>>(vars, paths, part);
   int st = check_launch("ls_moments");
   if (st) return st;
@@ -1428,7 +1434,7 @@ extern "C" int lmm_ls_moment_sums(int n_exercise, int paths, const float* d_vars
               "lmm_ls_moment_sums: workspace too small");
   cudaStream_t s = (cudaStream_t)stream;
   LsWs w = carve_ls(d_workspace, paths, n_exercise);
-  const int nblk = ls_gram_blocks();
+  const int nblk = moment_blocks(paths);
   ls_moments_kernel<<<dim3(nblk, n_exercise), 256, 0, s>>>(d_vars, paths, w.mom);
   int st = check_launch("ls_moments");
   if (st) return st;

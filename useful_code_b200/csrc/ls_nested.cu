@@ -226,7 +226,7 @@ __device__ bool grid_wait(unsigned int* counter, unsigned gen, int* ok_s) {
     __threadfence();
     atomicAdd(counter, 1u);
     int ok = 0;
-    for (int i = 0; i < (1 << 22) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
+    for (int i = 0; i < (1 << 25) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
     __threadfence();
     *ok_s = ok;
   }
