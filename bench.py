@@ -601,7 +601,7 @@ def run_b200(args) -> int:
         per_path = json.loads(tf.read_text()).get(f"fused_evolve_{args.config}_bytes_per_path")
         if per_path is not None and t_first is not None:
             traffic = per_path * Preg
-    kname = "tc_evolve_kernel" if tensor else "fused_evolve_kernel"
+    kname = "tc_evolve_kernel" if tensor else "fused_pairs_kernel"
     roofline = {"bound": "fp32", "kernel": f"{kname} (first pass)",
                 "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp32_peak, "traffic": traffic,

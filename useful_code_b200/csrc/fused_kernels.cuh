@@ -8,6 +8,7 @@
 // IEEE-accurate library forms and serve as the plain-FP32 reference of the
 // same arithmetic.
 #pragma once
+#include <algorithm>
 #include <type_traits>
 #include "lmm_common.cuh"
 #include "lmm_device.cuh"
@@ -155,49 +156,115 @@ __device__ __forceinline__ float2 icdf_sb_fast2(uint32_t va, uint32_t vb) {
 // has the same low bits of n, so it differs by Gray bit 6 and the one upper
 // bit in which gray(h + 1) differs from gray(h): one more XOR with a word
 // that is stored beside the upper XOR.  A pair of points costs three
-// shared-memory reads, with no data-dependent branch.  Points are generated
-// kVarBatch stages at a time (independent work for the scheduler), then
-// folded into the bridge, whose S points per path live in shared memory,
-// both paths of a thread in one packed FP32x2 value: the stage's weights and
-// offsets, the addressing and the loop control are read once per pair.
-// Output [step][factor][path] increments.
+// shared-memory reads, with no data-dependent branch.
 //
-// Bound by the shared-memory loads and their latency (the 3.4 GB of output
-// at 2^20 paths, 80 steps and 10 factors take 0.5 ms).  Against one path per
-// thread and one tile of 128 per CTA: 1.79 -> 1.68 ms there, 138 -> 115 us at
-// 300,001 paths, 40 steps and 5 factors, 1.18 -> 1.16 ms at 200,003 paths, 120
-// steps and 15 factors (where one CTA fills an SM's shared memory).
+// The bridge runs depth first over its tree of intervals instead of level by
+// level: a point's two neighbours are then its ancestors, and the points come
+// out from left to right, each increment as soon as its point's left subtree
+// is done.  Only the ancestors of the current point are held, one row per
+// depth (at most ten rows for 128 steps, against one per step), so an SM's
+// shared memory holds as many CTAs as the registers allow instead of two.
+// The host lists the points in that order (make_var_plan); every point is the
+// same combination of the same values.  Both paths of a thread run in one
+// packed FP32x2 value, so the point's weights and offsets, the addressing and
+// the loop control are read once per pair; normals are generated kVarBatch
+// points at a time (independent work for the scheduler).  Output
+// [step][factor][path] increments.
+//
+// Bound by instruction issue and the shared-memory reads (the 3.4 GB of
+// output at 2^20 paths, 80 steps and 10 factors take 0.5 ms).  One path per
+// thread level by level, two paths so, and this form: 1.79, 1.68, 1.17 ms
+// there; 200,003 paths, 120 steps, 15 factors 1.18, 1.16, 0.59 ms (one CTA per
+// SM level by level); 300,001 paths, 40 steps, 5 factors 141, 117, 114 us.
 // ---------------------------------------------------------------------------
 constexpr int kVarBlock = 128;
 constexpr int kVarTile = 2 * kVarBlock;  // paths per tile
 constexpr int kVarBatch = 8;
 constexpr int kVarTiles = 8;  // most tiles per CTA
 
+// The bridge's points in depth-first order: weights, rows of the neighbours
+// and the point itself (row `rows` - 1 stays zero: the neighbour of a point
+// that has none), how many points come out after it, and the Sobol dimension
+// of its normal per factor.  out_row: the row of each point in the order of
+// the steps.
+struct VarPlan {
+  int steps, factors, rows;
+  float lw[kMaxSteps], rw[kMaxSteps], sd[kMaxSteps];
+  unsigned char left[kMaxSteps], right[kMaxSteps], target[kMaxSteps];
+  unsigned char emits[kMaxSteps], out_row[kMaxSteps];
+  unsigned short dim[kMaxFactors * kMaxSteps];  // [factor][point]
+};
+
+inline void make_var_plan(const BridgePlan& b, VarPlan* v) {
+  const int S = b.steps;
+  int stage_of[kMaxSteps];
+  for (int i = 0; i < S; ++i) stage_of[b.bidx[i]] = i;
+  v->steps = S;
+  v->factors = b.factors;
+  int count = 0, depth_max = 0, row_of[kMaxSteps];
+  // point p at `depth`, neighbours' points l and r (-1: none)
+  auto put = [&](int p, int depth, int l, int r) {
+    const int i = stage_of[p], k = count++;
+    v->lw[k] = l >= 0 ? b.lw[i] : 0.0f;
+    v->rw[k] = r >= 0 ? b.rw[i] : 0.0f;
+    v->sd[k] = b.sd[i];
+    v->left[k] = l >= 0 ? (unsigned char)row_of[l] : 255;
+    v->right[k] = r >= 0 ? (unsigned char)row_of[r] : 255;
+    v->target[k] = (unsigned char)depth;
+    v->emits[k] = 0;
+    for (int f = 0; f < b.factors; ++f)
+      v->dim[f * kMaxSteps + k] = (unsigned short)b.alloc[f * S + i];
+    row_of[p] = depth;
+    depth_max = std::max(depth_max, depth);
+    return k;
+  };
+  int out = 0, last = put(S - 1, 0, -1, -1);  // the terminal point
+  // the points strictly between l and r
+  auto fill = [&](auto&& self, int l, int r, int depth) -> void {
+    if (r - l < 2) return;
+    const int m = l + 1 + ((r - 2 - l) >> 1);
+    last = put(m, depth, l, r);
+    self(self, l, m, depth + 1);
+    ++v->emits[last];
+    v->out_row[out++] = (unsigned char)depth;
+    self(self, m, r, depth + 1);
+  };
+  fill(fill, -1, S - 1, 1);
+  ++v->emits[last];
+  v->out_row[out] = 0;
+  v->rows = depth_max + 2;
+  for (int k = 0; k < S; ++k) {
+    if (v->left[k] == 255) v->left[k] = (unsigned char)(v->rows - 1);
+    if (v->right[k] == 255) v->right[k] = (unsigned char)(v->rows - 1);
+  }
+}
+
 __global__ void __launch_bounds__(kVarBlock)
     variates_kernel(int paths, uint32_t first_index, int tiles,
                     const uint32_t* __restrict__ dirs,
                     const uint32_t* __restrict__ scr, int scr_dims,
                     float* __restrict__ out,
-                    const __grid_constant__ BridgePlan plan) {
+                    const __grid_constant__ VarPlan plan) {
   constexpr int T = kVarBlock;
   constexpr int kRow = T * (int)sizeof(float2);  // bytes of a bridge row
   const int S = plan.steps, F = plan.factors;
-  // shared memory (variates_smem_bytes): the bridge points W[S + 1][T]
-  // (row S stays zero: the left neighbour of a point that has none), the
-  // bridge plan per construction stage as {lw, rw, sd} weights and
-  // {left row, right row, target row} byte offsets into W, and the
-  // Sobol tables up[2][S], lo4[S][17], hi3[S][9] (rows padded by one word,
-  // so that the one-thread-per-dimension stores hit distinct banks)
+  // shared memory (variates_smem_bytes): the rows of bridge points W[rows][T],
+  // the plan per point as {lw, rw, sd} weights with the points to put out and
+  // {left row, right row, target row} byte offsets into W, the rows of the
+  // points in the order of the steps, and the Sobol tables up[2][S],
+  // lo4[S][17], hi3[S][9] (rows padded by one word, so that the
+  // one-thread-per-dimension stores hit distinct banks)
   extern __shared__ __align__(16) float var_sm[];
   float2* W = reinterpret_cast<float2*>(var_sm);
-  float4* bw_s = reinterpret_cast<float4*>(W + (size_t)(S + 1) * T);
+  float4* bw_s = reinterpret_cast<float4*>(W + (size_t)plan.rows * T);
   int4* bo_s = reinterpret_cast<int4*>(bw_s + S);
   uint2* up_s = reinterpret_cast<uint2*>(bo_s + S);  // {upper XOR, second point's XOR}
   uint32_t* lo4_s = reinterpret_cast<uint32_t*>(up_s + 2 * S);
   uint32_t* hi3_s = lo4_s + 17 * S;
+  int* out_s = reinterpret_cast<int*>(hi3_s + 9 * S);  // byte offsets
   const int tid = threadIdx.x;
   const int f = blockIdx.y;
-  const int* alloc = plan.alloc + f * S;
+  const unsigned short* dim = plan.dim + f * kMaxSteps;
   int p0 = blockIdx.x * tiles * kVarTile;
   uint32_t h0 = (first_index + (uint32_t)p0) >> 7;
   // the second points' word for upper index h: Gray bit 6 and the bit that
@@ -211,7 +278,7 @@ __global__ void __launch_bounds__(kVarBlock)
   // and the two low tables, each entry the previous one with its lowest set
   // bit cleared, XOR that bit's direction number
   for (int i = tid; i < S; i += T) {
-    const int d = alloc[i];
+    const int d = dim[i];
     const uint32_t* v = dirs + 32 * d;
     uint32_t g = h0 ^ (h0 >> 1), x = 0;
     while (g) {
@@ -238,19 +305,13 @@ __global__ void __launch_bounds__(kVarBlock)
     for (int e = 0; e < 16; ++e) l4[e] = t4[e];
 #pragma unroll
     for (int e = 0; e < 8; ++e) h3[e] = t3[e];
-    // stage 0 is the terminal point W_S = sd_0 z (row S - 1); a stage
-    // without a left neighbour reads the zero row S with weight 0
-    const bool first = i == 0;
-    const int jl = first ? 0 : plan.left[i];
-    bw_s[i] = make_float4(jl != 0 ? plan.lw[i] : 0.0f, first ? 0.0f : plan.rw[i], plan.sd[i],
-                          0.0f);
-    bo_s[i] = make_int4((jl != 0 ? jl - 1 : S) * kRow, (first ? S : plan.right[i]) * kRow,
-                        (first ? S - 1 : plan.bidx[i]) * kRow, 0);
+    bw_s[i] = make_float4(plan.lw[i], plan.rw[i], plan.sd[i], __int_as_float(plan.emits[i]));
+    bo_s[i] = make_int4(plan.left[i] * kRow, plan.right[i] * kRow, plan.target[i] * kRow, 0);
+    out_s[i] = plan.out_row[i] * kRow;
   }
-  W[(size_t)S * T + tid] = dup2(0.0f);
+  W[(size_t)(plan.rows - 1) * T + tid] = dup2(0.0f);
   __syncthreads();
-  float2* w = W + tid;
-  char* wb = reinterpret_cast<char*>(w);
+  char* wb = reinterpret_cast<char*>(W + tid);
   for (int t = 0; t < tiles && p0 < paths; ++t) {
     const int p = p0 + tid;
     const uint32_t n = first_index + (uint32_t)p;
@@ -259,8 +320,13 @@ __global__ void __launch_bounds__(kVarBlock)
     const uint2* up_t = up_s + ((n >> 7) - h0) * S;
     const uint32_t* lo_t = lo4_s + (glo & 15u);
     const uint32_t* h3_t = hi3_s + (glo >> 4);
-    // one batch of kVarBatch stages from i0; FULL: all of them exist (no
-    // clamp of the stage index, no guard on the bridge step)
+    const bool both = p + T < paths;
+    float2 prev = dup2(0.0f);
+    float* o = out + (size_t)f * paths + p;
+    const size_t o_step = (size_t)F * paths;
+    const int* next_out = out_s;
+    // one batch of kVarBatch points from i0; FULL: all of them exist (no
+    // clamp of the index, no guard on the bridge step)
     auto batch = [&](int i0, auto full_tag) {
       constexpr bool FULL = decltype(full_tag)::value;
       float2 z[kVarBatch];
@@ -277,11 +343,18 @@ __global__ void __launch_bounds__(kVarBlock)
         if (FULL || i < S) {
           const float4 bw = bw_s[i];
           const int4 bo = bo_s[i];
-          // bo: byte offsets of the stage's rows (no index scaling per access)
+          // bo: byte offsets of the rows (no index scaling per access)
           float2 y = __fmul2_rn(dup2(bw.x), *reinterpret_cast<const float2*>(wb + bo.x));
           y = __ffma2_rn(dup2(bw.y), *reinterpret_cast<const float2*>(wb + bo.y), y);
           y = __ffma2_rn(dup2(bw.z), z[k], y);
           *reinterpret_cast<float2*>(wb + bo.z) = y;
+          // the points whose left subtree this one completes
+          for (int c = __float_as_int(bw.w); c > 0; --c, ++next_out, o += o_step) {
+            const float2 cur = *reinterpret_cast<const float2*>(wb + *next_out);
+            o[0] = cur.x - prev.x;
+            if (both) o[T] = cur.y - prev.y;
+            prev = cur;
+          }
         }
       }
     };
@@ -289,24 +362,13 @@ __global__ void __launch_bounds__(kVarBlock)
       int i0 = 0;
       for (; i0 + kVarBatch <= S; i0 += kVarBatch) batch(i0, std::true_type());
       if (i0 < S) batch(i0, std::false_type());
-      float2 prev = dup2(0.0f);
-      float* o = out + (size_t)f * paths + p;
-      const size_t o_step = (size_t)F * paths;
-      const bool both = p + T < paths;
-#pragma unroll 4
-      for (int s = 0; s < S; ++s, o += o_step) {
-        const float2 cur = w[s * T];
-        o[0] = cur.x - prev.x;
-        if (both) o[T] = cur.y - prev.y;
-        prev = cur;
-      }
     }
     p0 += kVarTile;
     h0 += 2u;
     if (t + 1 < tiles && p0 < paths) {  // the next tile's upper XORs
       __syncthreads();
       for (int i = tid; i < S; i += T) {
-        const uint32_t* v = dirs + 32 * alloc[i];
+        const uint32_t* v = dirs + 32 * dim[i];
         const uint2 last = up_s[S + i];  // of h0 - 1
         const uint32_t v6 = __ldg(v + 6);
         const uint32_t x = last.x ^ last.y ^ v6;
@@ -319,10 +381,11 @@ __global__ void __launch_bounds__(kVarBlock)
   }
 }
 
-// Shared memory of variates_kernel for S bridge stages.
-inline size_t variates_smem_bytes(int S) {
-  return (size_t)(S + 1) * kVarBlock * sizeof(float2) + (size_t)S * (sizeof(float4) + sizeof(int4)) +
-         (size_t)S * (2 * sizeof(uint2) + (17 + 9) * sizeof(uint32_t));
+// Shared memory of variates_kernel.
+inline size_t variates_smem_bytes(const VarPlan& p) {
+  return (size_t)p.rows * kVarBlock * sizeof(float2) +
+         (size_t)p.steps * (sizeof(float4) + sizeof(int4) + 2 * sizeof(uint2) +
+                            (17 + 9 + 1) * sizeof(uint32_t));
 }
 
 }  // namespace lmm

@@ -567,20 +567,22 @@ int launch_variates(const Validated& v, const lmm_model* m, int P, uint32_t off,
   TRY(make_bridge_plan(v.n, v.F, nullptr, &plan));
   LMM_REQUIRE((uint64_t)off + (uint64_t)P + 1u < (1ull << 31),
               "pipeline: Sobol point index must stay below 2^31");
-  const size_t smem = variates_smem_bytes(v.n);
+  VarPlan vp;
+  make_var_plan(plan, &vp);
+  const size_t smem = variates_smem_bytes(vp);
   TRY(check_cuda(cudaFuncSetAttribute(variates_kernel,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem),
                  "variates: smem attribute"));
   // several tiles per CTA, so that the Sobol tables and the bridge plan are
-  // built once for them, while the grid still holds every SM's CTAs (two at
-  // 80 steps) several times over
+  // built once for them, while the grid still holds every SM's CTAs (eight or
+  // so) several times over
   const int all = div_up(P, kVarTile);
-  const int tiles = std::max(1, std::min(kVarTiles, all * v.F / (16 * sm_count())));
+  const int tiles = std::max(1, std::min(kVarTiles, all * v.F / (32 * sm_count())));
   dim3 grid(div_up(all, tiles), v.F);
   variates_kernel<<<grid, kVarBlock, smem, s>>>(P, off + 1u, tiles, m->d_directions,
                                                 m->d_scramblers, m->scramble_dims,
-                                                out, plan);
+                                                out, vp);
   return check_launch("variates_kernel");
 }
 
