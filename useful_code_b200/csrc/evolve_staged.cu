@@ -1,5 +1,5 @@
 // evolve_staged.cu — the plain-FP32 staged chain: correlation + fixed drift,
-// one predictor-corrector launch per step, then discount ratios, coterminal
+// the predictor-corrector steps (one launch), then discount ratios, coterminal
 // annuities and swap rates, spot numeraires and the gather kernels.  Each
 // stage reads and writes full [step][rate][path] tensors in HBM, as the
 // reference's staged chain does (LMM_evolver_full.cu:154-262,

@@ -4,7 +4,7 @@
 // Staged mode runs the reference's chain stage by stage through full
 // [step][rate][path] tensors (LMM_evolver_full.cu:154-262 and the pass loops
 // of kooexample/bermudanIRDPricer.cu:650-947,1201-1480): Sobol -> scramble ->
-// inverse normal -> bridge -> correlate+drift -> one PC launch per step ->
+// inverse normal -> bridge -> correlate+drift -> PC steps (one launch) ->
 // discount ratios -> annuities -> swap rates -> numeraires -> extraction ->
 // basis variables / exercise values / coupons -> partial discounting ->
 // aggregation.
