@@ -190,8 +190,9 @@ int lmm_fused_evolve(const lmm_model* model, const lmm_product* product,
 /* lmm_fused_evolve's rule pass (the second pass of BermudanMultiLSPricer-
  * Example, kooexample/bermudanIRDPricer.cu:1091-1483) with a nested or
  * shifted rule (NULL for the European strip and the TARN), run as a chain of
- * launches over segments of segment_steps steps (< 1: the library default,
- * 8; >= rates: one launch): after each segment the paths that have
+ * launches over segments of segment_steps steps (< 1: the library's choice,
+ * 8 or 16 steps, or one launch when few paths leave the GPU idle anyway; >=
+ * rates: one launch): after each segment the paths that have
  * exercised are dropped and the survivors are packed, so later steps run on
  * full warps.  Payoffs are bit-identical to lmm_fused_evolve's.  The
  * workspace holds two survivor buffers of about (rates + 7) x 4 B per path

@@ -549,11 +549,26 @@ int fused_segments(const Validated& v, int P, const float* Z, const lmm_model* m
   return LMM_OK;
 }
 
-// segment_steps < 1: the library's kSegSteps; >= rates: one launch.
+// Steps per segment unless the caller asks otherwise.  Dropping exercised
+// paths pays where the SMs are full; with at most one CTA per SM a launch
+// lasts as long as its longest path anyway, and every further launch adds its
+// gap and its survivors' way through memory: one launch there, twice as long
+// segments up to four CTAs per SM.  Measured (8, 16 steps, one launch): 80
+// rates, 10 factors 0.60, 0.53, 0.47 ms at 18,944 paths, 0.87, 0.81, 0.82 at
+// 65,536, 1.12, 1.08, 1.09 at 95,000; 120 rates, 15 factors 1.25, 1.15, 1.01 at
+// 18,944, 1.33, 1.22, 1.45 at 30,000, 1.83, 1.80, 2.06 at 65,536, 2.33, 2.39,
+// 2.83 at 95,000; 40 rates, 5 factors 0.21, 0.18, 0.16 at 18,944, 0.26, 0.23,
+// 0.25 at 65,536.
+int default_segment(const Validated& v, int P) {
+  const int ctas = div_up(P, kFusedBlock);
+  return ctas <= sm_count() ? v.n : ctas <= 4 * sm_count() ? 2 * kSegSteps : kSegSteps;
+}
+
+// segment_steps < 1: default_segment; >= rates: one launch.
 int fused_price(const Validated& v, int P, const float* Z, const lmm_model* m,
                 const LsRuleView& rule, Carver& c, int segment_steps, float* payoff,
                 cudaStream_t s) {
-  const int len = segment_steps < 1 ? kSegSteps : segment_steps;
+  const int len = segment_steps < 1 ? default_segment(v, P) : segment_steps;
   if (!segmentable(v) || len >= v.n)
     return launch_fused<kModeRule>(v, P, Z, m, rule, P, 0, nullptr, nullptr, nullptr,
                                    nullptr, payoff, s);
@@ -951,8 +966,10 @@ extern "C" int lmm_fused_price(const lmm_model* model, const lmm_product* produc
   LMM_REQUIRE(paths >= 1 && d_variates && d_payoff, "lmm_fused_price: bad arguments");
   LsRuleView view = ls_rule_view(nullptr, nullptr, nullptr);
   if (!no_exercise(product->kind)) TRY(rule_from_abi(rule, &view, "lmm_fused_price"));
+  // a chain's workspace is asked for by the caller's choice (one launch needs
+  // none), not by the library's for this number of paths
   const int len = segment_steps < 1 ? kSegSteps : segment_steps;
-  const size_t need = len < v.n ? seg_ws_bytes(v, paths) : 0;  // one launch needs none
+  const size_t need = len < v.n ? seg_ws_bytes(v, paths) : 0;
   LMM_REQUIRE(need == 0 || (d_workspace && workspace_bytes >= need),
               "lmm_fused_price: workspace %zu < %zu", workspace_bytes, need);
   Carver c{(char*)d_workspace};
@@ -1046,10 +1063,11 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
   // alias the recompute buffers of the reverse sweep, unused until then.
   const LsRuleView rule = ls_rule_view(d_beta, d_means, d_sds);
   const size_t recompute_bytes = greeks_seg_floats(n, P, k) * sizeof(float);
-  if (segmentable(v) && kSegSteps < n && seg_ws_bytes(v, P) <= recompute_bytes) {
+  const int seg_steps = default_segment(v, P);
+  if (segmentable(v) && seg_steps < n && seg_ws_bytes(v, P) <= recompute_bytes) {
     Carver sc{(char*)b.seg[0]};
     const SegBufs sb = carve_seg(sc, v, P);
-    TRY(fused_segments<kModeRecord>(v, P, b.Z, model, rule, sb, kSegSteps, b.payoff, s, rec));
+    TRY(fused_segments<kModeRecord>(v, P, b.Z, model, rule, sb, seg_steps, b.payoff, s, rec));
   } else {
     TRY(launch_fused<kModeRecord>(v, P, b.Z, model, rule, P, 0, nullptr, nullptr, nullptr,
                                   nullptr, b.payoff, s, rec));
