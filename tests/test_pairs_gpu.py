@@ -88,3 +88,59 @@ def test_variates_pieces(cuda, n, F, P, offset):
         piece = torch.empty(n, F, size, device="cuda")
         call("lmm_fused_variates", addr, size, offset + lo, dp(piece), stream_handle())
         assert torch.equal(whole[:, :, lo:lo + size], piece), lo
+
+
+@pytest.mark.parametrize("n", [2, 3, 4, 5, 7, 8, 9, 16, 31, 33, 63, 64, 65, 100, 127, 128])
+def test_variates_depth_first_bridge(cuda, n):
+    """Every tree shape of the depth-first bridge against the level-by-level
+    construction in FP64 on exact normals.  Bridge values reach 6 sqrt(128) =
+    68; an FP32 combination rounds them by up to 68 * 2^-23 = 8e-6 per level
+    (at most eight levels) and the rational inverse normal is within 7e-7
+    relative of the exact one: 1e-4 bounds the difference of two points."""
+    from scipy.special import ndtri
+
+    from useful_code_b200 import market as mk
+    from useful_code_b200._lib import call
+    from useful_code_b200.pricer import LmmModel, LmmProduct, dp, stream_handle  # noqa: F401
+
+    F, P, offset = 2, 300, 1000
+    pipe = pipeline("c3", n, F)
+    n_, alloc = n, np.zeros(F * n, np.int32)
+    model = pipe.model
+    taus = np.full(n_, 0.25, np.float32)
+    disp = np.full(n_, 0.015, np.float32)
+    f0 = np.full(n_, 0.04, np.float32)
+    dirs = mk.sobol_directions(F * n_)
+    scr = mk.scramblers(7, F * n_)
+    d_dirs = torch.from_numpy(dirs.astype(np.int32)).cuda()
+    d_scr = torch.from_numpy(scr.astype(np.int32)).cuda()
+    vp = ctypes.c_void_p
+    m = LmmModel(n_, F, vp(taus.ctypes.data), vp(disp.ctypes.data), vp(f0.ctypes.data),
+                 model.d_A, model.d_fixed_drifts, dp(d_dirs), dp(d_scr), F * n_, 10.0)
+    out = torch.empty(n_, F, P, device="cuda")
+    call("lmm_fused_variates", ctypes.addressof(m), P, offset, dp(out), stream_handle())
+    lw, rw, sd = (np.zeros(n_) for _ in range(3))
+    left, right, bidx = (np.zeros(n_, np.int32) for _ in range(3))
+    call("lmm_bridge_tables_host", n_, *(vp(a.ctypes.data)
+                                         for a in (lw, rw, sd, left, right, bidx)))
+    call("lmm_bridge_allocate_diagonal", F, n_, vp(alloc.ctypes.data))
+    idx = np.arange(1 + offset, 1 + offset + P, dtype=np.uint64)
+    gray = idx ^ (idx >> np.uint64(1))
+    ref = np.zeros((n_, F, P))
+    for f in range(F):
+        W = np.zeros((n_, P))
+        for i in range(n_):
+            d = alloc.reshape(F, n_)[f, i]
+            x = np.full(P, scr[d], np.uint32)
+            for b in range(12):
+                x ^= np.where((gray >> np.uint64(b)) & np.uint64(1), dirs[d, b], 0).astype(
+                    np.uint32)
+            z = ndtri(np.clip(x.astype(np.float64), 1.0, None) * 2.0 ** -32)
+            y = sd[i] * z
+            if i > 0:
+                y += rw[i] * W[right[i]]
+                if left[i] > 0:
+                    y += lw[i] * W[left[i] - 1]
+            W[bidx[i]] = y
+        ref[:, f] = np.diff(W, axis=0, prepend=0.0)
+    assert np.max(np.abs(out.cpu().numpy() - ref)) < 1e-4

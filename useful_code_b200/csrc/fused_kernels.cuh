@@ -90,7 +90,7 @@ struct SegIO {
 };
 
 // Continuation estimate of the frozen rule at exercise date e (depth chain
-// and Andersen shift of ls_chain_estimate).
+// and Andersen shift of ls_chain_estimates).
 __device__ __forceinline__ double rule_estimate(const RuleConst& rc, int e, const float* v,
                                                 float exv, const LsRuleView& rule) {
   const float v1[1][kMaxVars] = {{v[0], v[1], v[2]}}, ex1[1] = {exv};
@@ -101,27 +101,10 @@ __device__ __forceinline__ double rule_estimate(const RuleConst& rc, int e, cons
 }
 
 // Shaw–Brickman inverse normal on the exact tail probability
-// (icdf_sb_tails) with the hardware log and reciprocal approximations.
-__device__ __forceinline__ float icdf_sb_fast(uint32_t vi) {
-  float sgn;
-  const float t = icdf_tail_t(vi, &sgn);
-  const float z = -log_ftz(t);
-  // numerator p and denominator q by one Horner recurrence on the pair
-  // (p, q): each packed FMA rounds as the scalar FMA of the nested form
-  const float2 z2 = make_float2(z, z);
-  float2 pq = __ffma2_rn(make_float2(4.744820732427972462e-6f, 0.00010590620919921025259f), z2,
-                         make_float2(0.0020751409553756572917f, 0.0120098270559197768f));
-  pq = __ffma2_rn(pq, z2, make_float2(0.087403248265958578062f, 0.23668431621373705623f));
-  pq = __ffma2_rn(pq, z2, make_float2(0.80002295072483916762f, 1.2499328117341603014f));
-  pq = __ffma2_rn(pq, z2, make_float2(1.9797154223229267471f, 2.0795584360534589311f));
-  pq = __ffma2_rn(pq, z2, make_float2(1.2533136835212087879f, 1.0f));
-  return sgn * ((z * pq.x) * rcp_ftz(pq.y));
-}
-
-// icdf_sb_fast for two points per thread, each half with icdf_sb_fast's own
-// roundings: the numerator and denominator recurrences run on the pair of
-// points (no packing of a point's own numerator and denominator), and the
-// sign, +1 for integers from 2^31, is set as a bit.
+// (icdf_sb_tails) with the hardware log and reciprocal approximations, for two
+// points per thread: the numerator and denominator recurrences run on the
+// packed pair, each half with the roundings of the scalar FMAs, and the sign,
+// +1 for integers from 2^31, is set as a bit.
 __device__ __forceinline__ float2 icdf_sb_fast2(uint32_t va, uint32_t vb) {
   auto tail = [](uint32_t v) {
     return fmaxf(__uint2float_rn(min(v, 0u - v)) * 4.656612873077392578125e-10f,
@@ -201,7 +184,7 @@ inline void make_var_plan(const BridgePlan& b, VarPlan* v) {
   for (int i = 0; i < S; ++i) stage_of[b.bidx[i]] = i;
   v->steps = S;
   v->factors = b.factors;
-  int count = 0, depth_max = 0, row_of[kMaxSteps];
+  int count = 0, depth_max = 0, row_of[kMaxSteps] = {};
   // point p at `depth`, neighbours' points l and r (-1: none)
   auto put = [&](int p, int depth, int l, int r) {
     const int i = stage_of[p], k = count++;

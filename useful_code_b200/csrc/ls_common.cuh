@@ -144,12 +144,6 @@ __device__ __forceinline__ void ls_powers(const float* x, float (&pw)[kMaxVars][
   }
 }
 
-// Continuation estimate of a frozen rule at date e for basis variables v
-// and exercise value exv: the depth chain of MultiLSExerciseStrategy::decide
-// (gold/MultiLS_regression.h:190-231) and updateDeflatedNextStepValuesMulti_
-// gold (:42-99): regression d + 1 is used while the net value estimate -
-// exv of regression d lies strictly inside d's cuts.  The caller exercises
-// when exv > estimate.
 // sum_k phi_k(x) b[k] with x standardised by mean / sd (null: raw).
 __device__ __forceinline__ double ls_row_estimate(const double* b, const float* mean,
                                                   const float* sd, int nvars, int nbasis,
@@ -171,23 +165,6 @@ __device__ __forceinline__ double ls_row_estimate(const double* b, const float* 
 #pragma unroll
   for (int k = 0; k < kMaxBasis; ++k)
     if (k < nbasis) est += (double)ls_monomial(pw, mono[k]) * b[k];
-  return est;
-}
-
-__device__ __forceinline__ double ls_chain_estimate(const LsRuleView& r, int e, int nvars,
-                                                    int nbasis,
-                                                    const unsigned char (*mono)[kMaxVars],
-                                                    const float* v, float exv) {
-  double est = 0.0;
-  for (int d = 0; d < r.depth; ++d) {
-    const size_t row = (size_t)e * r.depth + d;
-    est = (r.shifts ? (double)r.shifts[e] : 0.0) +
-          ls_row_estimate(r.beta + row * kMaxBasis, r.means ? r.means + row * kMaxVars : nullptr,
-                          r.means ? r.sds + row * kMaxVars : nullptr, nvars, nbasis, mono, v);
-    if (d + 1 >= r.depth || !r.cuts) break;
-    const double net = est - (double)exv;
-    if (!(net > r.cuts[row * 2] && net < r.cuts[row * 2 + 1])) break;
-  }
   return est;
 }
 
@@ -221,7 +198,13 @@ __device__ __forceinline__ void ls_row_estimate_known(const double* b, const flo
   }
 }
 
-// ls_chain_estimate for H paths per thread; kind: the date's basis kind.
+// Continuation estimate of a frozen rule at date e for basis variables v
+// and exercise value exv: the depth chain of MultiLSExerciseStrategy::decide
+// (gold/MultiLS_regression.h:190-231) and updateDeflatedNextStepValuesMulti_
+// gold (:42-99): regression d + 1 is used while the net value estimate -
+// exv of regression d lies strictly inside d's cuts.  The caller exercises
+// when exv > estimate.
+// H paths per thread; kind: the date's basis kind.
 template <int H>
 __device__ __forceinline__ void ls_chain_estimates(const LsRuleView& r, int e, int kind,
                                                    int nvars, int nbasis,
