@@ -118,6 +118,23 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// One thread's part of a barrier between the CTAs of a cooperative grid: adds
+// its arrival to *counter and waits until it has reached `want`.  Release and
+// acquire at device scope order the CTA's earlier writes (joined by a CTA
+// barrier before the call) before the other CTAs' later reads (after one),
+// without the full fences around a plain atomic.  The wait is bounded (about
+// 20 s): false when it ran out, which it cannot while every CTA is resident
+// and arrives.
+__device__ __forceinline__ bool grid_arrive_wait(unsigned int* counter, unsigned want) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+  for (int i = 0; i < (1 << 25); ++i) {
+    unsigned c;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(counter) : "memory");
+    if (c >= want) return true;
+  }
+  return false;
+}
+
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }

@@ -816,12 +816,7 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
     __syncthreads();
     if (tid == 0) {
       const unsigned want = (unsigned)(E - e) * gridDim.x;
-      __threadfence();
-      atomicAdd(counter, 1u);
-      int ok = 0;
-      for (int i = 0; i < (1 << 25) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
-      __threadfence();
-      ok_s = ok;
+      ok_s = grid_arrive_wait(counter, want);
     }
     __syncthreads();
     if (!ok_s) return false;  // never while every CTA is resident

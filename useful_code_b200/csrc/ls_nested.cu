@@ -222,13 +222,7 @@ __device__ void sel_advance(SelState& shared, const double* thr, const int* cnt)
 __device__ bool grid_wait(unsigned int* counter, unsigned gen, int* ok_s) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    const unsigned want = gen * gridDim.x;
-    __threadfence();
-    atomicAdd(counter, 1u);
-    int ok = 0;
-    for (int i = 0; i < (1 << 25) && !ok; ++i) ok = *(volatile unsigned int*)counter >= want;
-    __threadfence();
-    *ok_s = ok;
+    *ok_s = grid_arrive_wait(counter, gen * gridDim.x);
   }
   __syncthreads();
   return *ok_s != 0;
