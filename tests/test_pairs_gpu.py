@@ -144,3 +144,24 @@ def test_variates_depth_first_bridge(cuda, n):
             W[bidx[i]] = y
         ref[:, f] = np.diff(W, axis=0, prepend=0.0)
     assert np.max(np.abs(out.cpu().numpy() - ref)) < 1e-4
+
+
+def test_tensor_memory_handed_over(cuda):
+    """CTAs of two launches on two streams share the SMs and take over one
+    another's tensor-memory columns (a few hundred CTAs each, three per SM):
+    every pass gives the bits it gives alone."""
+    pipes = [pipeline("c3", 80, 10), pipeline("c3", 80, 10)]
+    rule = pipes[0].regress(pipes[0].first_pass(8192, 0))
+    P = 150001
+    alone = pipes[0].second_pass(P, 4242, rule)
+    first = pipes[1].first_pass(P, 4242)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(4):
+        with torch.cuda.stream(streams[0]):
+            pay = pipes[0].second_pass(P, 4242, rule)
+        with torch.cuda.stream(streams[1]):
+            ls = pipes[1].first_pass(P, 4242)
+        torch.cuda.synchronize()
+        assert torch.equal(pay, alone)
+        assert torch.equal(ls.vars, first.vars) and torch.equal(ls.num, first.num)

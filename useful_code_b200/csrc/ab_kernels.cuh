@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
     float2 x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) x[j] = start_rate(r + j);
+    __syncwarp();
     tmem_st8(lr.tmem + 2 * (r - nt0), x);
   }
   const float N0 = __ldg(ckptN + (size_t)s0 * a.K + p);
@@ -203,9 +204,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
       red_s[1][2 * warp + h] = s2;
     }
   }
-  tmem_fence_before();
-  __syncthreads();
-  if (tmem_cols && warp == 0) tmem_dealloc(tmem_slot, tmem_cols);
+  tmem_free(lr.tmem, tmem_cols);  // and red_s is complete
   if ((tid & 63) == 0 && valid) {
     double t1 = 0.0, t2 = 0.0;
     for (int w = 0; w < kAbThreads / 32; ++w) {

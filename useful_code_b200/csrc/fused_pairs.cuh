@@ -163,6 +163,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
     float2 x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) x[j] = start_rate(r + j);
+    __syncwarp();
     tmem_st8(lr.tmem + 2 * (r - nt0), x);
   }
   if (resume) {
@@ -385,11 +386,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
       if (live[0]) row[slot[0]] = x.x;
       if (live[1]) row[slot[1]] = x.y;
     });
-    if (tmem_cols) {
-      tmem_fence_before();
-      __syncthreads();
-      if (warp == 0) tmem_dealloc(tmem_slot, tmem_cols);
-    }
+    tmem_free(lr.tmem, tmem_cols);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       if (live[h]) {
@@ -408,11 +405,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
     if (tid == 0) seg.out_count[blockIdx.x] = tot;
     return;
   }
-  if (tmem_cols) {
-    tmem_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_slot, tmem_cols);
-  }
+  tmem_free(lr.tmem, tmem_cols);
   // an exercise date at the last step: its curve is the one period
   if (pend[0] || pend[1]) {
     const float ann[2] = {mc.tau[n - 1] * pend_P1[0], mc.tau[n - 1] * pend_P1[1]};

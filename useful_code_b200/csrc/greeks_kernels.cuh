@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
     float2 x[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) x[j] = start_rate(r + j);
+    __syncwarp();
     tmem_st8(lr.tmem + 2 * (r - nt0), x);
   }
   float N[2], f_first[2] = {0.0f, 0.0f};
@@ -292,6 +293,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
             Prun = __fmul2_rn(Prun, make_float2(rcp_ftz(t.x), rcp_ftz(t.y)));
             ann = __ffma2_rn(dup2(mc.tau[r]), Prun, ann);
           }
+          __syncwarp();
         });
     f_first[0] = exp_ftz(ln_first.x) - mc.disp[s];
     f_first[1] = exp_ftz(ln_first.y) - mc.disp[s];
@@ -311,11 +313,7 @@ __global__ void __launch_bounds__(kPairThreads, PairShape<FT>::kCtas)
       info[(size_t)(2 * F + 2) * P + p[h]] = c ? (h ? ann.y : ann.x) : 0.0f;
     }
   }
-  if (tmem_cols) {
-    tmem_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_slot, tmem_cols);
-  }
+  tmem_free(lr.tmem, tmem_cols);
 }
 
 // ---------------------------------------------------------------------------

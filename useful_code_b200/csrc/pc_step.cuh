@@ -179,6 +179,7 @@ __host__ __device__ __forceinline__ uint32_t tmem_columns(int rows) {
 // starts no further CTA of the kernel (1 instead of 4 CTAs per SM measured
 // without it, 0.92 against 0.44 ms for 2^18 paths of 40 rates).
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
+  __syncwarp();  // whole warps only, after whatever per-path branches came before
   if (cols)
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(slot)),
@@ -186,15 +187,28 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t cols) {
                  : "memory");
   asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_dealloc(uint32_t tmem, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols)
-               : "memory");
-}
 __device__ __forceinline__ void tmem_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+// Frees the CTA's columns (`cols` may be 0); contains a CTA barrier, all
+// threads.  The last step's stores have no load behind them that would wait
+// for them, so every warp waits for its own here: once the columns are free,
+// another CTA of the SM may be given them.
+__device__ __forceinline__ void tmem_free(uint32_t tmem, uint32_t cols) {
+  if (cols) {
+    __syncwarp();
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    tmem_fence_before();
+  }
+  __syncthreads();
+  if (cols && threadIdx.x < 32) {
+    tmem_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols)
+                 : "memory");
+  }
 }
 __device__ __forceinline__ void tmem_st8(uint32_t a, const float2 (&x)[4]) {
   asm volatile(
@@ -230,6 +244,7 @@ struct LogRates {
     for (int r = s; r < nt0; ++r) fn(r, row[(r - s_begin) * T]);
     for (int r0 = nt0 + (max(s - nt0, 0) & ~3); r0 < n; r0 += 4) {
       float2 x[4];
+      __syncwarp();  // fn may branch per path
       tmem_ld8(tmem + 2 * (r0 - nt0), x);
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -241,7 +256,8 @@ struct LogRates {
 // One step: pc_rate2 over the rates s .. n - 1 of the log-rates lr (whole
 // warps).  As, fx: the step's rows, rate r at row r - s.  hook(r, g, gp, q,
 // ln): called per rate with pc_rate2's outputs and the new log-rates before
-// the cap.  Returns the new log-rates of rate s.
+// the cap; it leaves the warp whole (tensor memory is accessed by whole
+// warps).  Returns the new log-rates of rate s.
 template <int FM, int FP, int T, class Hook>
 __device__ __forceinline__ float2 pc_step2(const LogRates<T>& lr, int s, int n,
                                            const ModelConst& mc, const float* As,
@@ -254,6 +270,7 @@ __device__ __forceinline__ float2 pc_step2(const LogRates<T>& lr, int s, int n,
     hook(r, g, gp, q, lf);
     return cap2(lf, mc.cutoff);
   };
+  __syncwarp();  // per-path branches of the caller end here
   float2 lf0 = dup2(0.0f);
   float2* row = lr.row + (s - lr.s_begin) * T;
 #pragma unroll 4
