@@ -9,6 +9,7 @@ results are compared bit for bit.
 from __future__ import annotations
 
 import ctypes
+import threading
 from dataclasses import replace
 
 import numpy as np
@@ -165,3 +166,32 @@ def test_tensor_memory_handed_over(cuda):
         torch.cuda.synchronize()
         assert torch.equal(pay, alone)
         assert torch.equal(ls.vars, first.vars) and torch.equal(ls.num, first.num)
+
+
+def test_threads_price_at_once(cuda):
+    """Two host threads launch the same kernels with different amounts of
+    shared memory (the segments of a chain, models of other sizes): neither
+    takes away the other's, and each gets the payoffs it gets alone."""
+    P = 100003
+    pipes = [pipeline("c3", 80, 10), pipeline("c3", 128, 10)]
+    rules = [p.regress(p.first_pass(8192, 0)) for p in pipes]
+    alone = [p.second_pass(P, 4242, r) for p, r in zip(pipes, rules)]
+    torch.cuda.synchronize()
+    errors = []
+
+    def price(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(40):
+                    pay = pipes[k].second_pass(P, 4242, rules[k])
+                if not torch.equal(pay, alone[k]):
+                    errors.append(f"thread {k}: other payoffs")
+        except RuntimeError as e:
+            errors.append(f"thread {k}: {e}")
+
+    threads = [threading.Thread(target=price, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors

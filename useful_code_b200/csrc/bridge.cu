@@ -200,14 +200,8 @@ extern "C" int lmm_bridge_transform(const float* d_in, float* d_out, int paths,
   const int block = 128;
   const size_t smem = (size_t)(steps + 1) * block * sizeof(float) +
                       (size_t)steps * (sizeof(float4) + sizeof(int4) + sizeof(int));
-  if (smem > 48 * 1024) {
-    int s2 = check_cuda(cudaFuncSetAttribute(
-                            bridge_kernel,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)smem),
-                        "lmm_bridge_transform: smem attribute");
-    if (s2 != LMM_OK) return s2;
-  }
+  st = allow_smem((const void*)bridge_kernel, smem, "lmm_bridge_transform: smem attribute");
+  if (st != LMM_OK) return st;
   int gx = div_up(paths, block);
   int cap = sm_count() * 8;
   if (gx > cap) gx = cap;

@@ -57,6 +57,28 @@ int sm_count() {
   return cached[dev];
 }
 
+// A kernel's limit is one value for all threads of the process.  One made to
+// a launch's measure could be lowered by another thread's call between this
+// call and the launch, so it only ever goes to the device's most: every
+// thread that sets it sets the same value.
+int allow_smem(const void* kern, size_t bytes, const char* what) {
+  cudaFuncAttributes fa;
+  int st = check_cuda(cudaFuncGetAttributes(&fa, kern), what);
+  if (st || bytes <= (size_t)fa.maxDynamicSharedSizeBytes) return st;
+  int dev = 0, most = 0;
+  st = check_cuda(cudaGetDevice(&dev), what);
+  if (st) return st;
+  st = check_cuda(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev),
+                  what);
+  if (st) return st;
+  most -= (int)fa.sharedSizeBytes;
+  if (bytes > (size_t)most)
+    return fail(LMM_ECUDA, "%s: %zu bytes of shared memory, the device has %d", what, bytes,
+                most);
+  return check_cuda(
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most), what);
+}
+
 }  // namespace lmm
 
 extern "C" const char* lmm_last_error_string(void) { return lmm::g_last_error; }

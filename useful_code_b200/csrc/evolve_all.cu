@@ -151,9 +151,7 @@ extern "C" int lmm_evolve_pc_all(const float* h_initial_rates, const float* h_ta
   cudaStream_t s = (cudaStream_t)stream;
   const int grid = div_up(paths, kAllBlock);
   auto go = [&](auto kern) -> int {
-    int st = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem),
-                        "lmm_evolve_pc_all: smem attribute");
+    int st = allow_smem((const void*)kern, smem, "lmm_evolve_pc_all: smem attribute");
     if (st) return st;
     kern<<<grid, kAllBlock, smem, s>>>(paths, steps, d_variates, variates_layout, d_A,
                                        d_fixed_drifts, mc, al, d_rates, d_log_rates,

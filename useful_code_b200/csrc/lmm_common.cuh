@@ -32,6 +32,9 @@ int fail(int code, const char* fmt, ...);
 int check_launch(const char* what);
 int check_cuda(cudaError_t e, const char* what);
 
+// Lets launches of `kern` have `bytes` of dynamic shared memory.
+int allow_smem(const void* kern, size_t bytes, const char* what);
+
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
 // Number of SMs of the current device (cached per device).

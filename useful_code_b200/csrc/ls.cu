@@ -29,7 +29,6 @@
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
-#include <vector>
 
 using namespace lmm;
 
@@ -1025,28 +1024,6 @@ size_t ls_workspace_bytes(int paths, int n_ex) {
   return y + part + cnt + mom + red + 256;
 }
 
-// Raise the dynamic shared-memory limit of a date kernel instantiation
-// (once per instantiation and device) when its staged loop needs more than
-// the default 48 KB.
-template <class Kern>
-int ls_stage_attr(Kern kern, size_t bytes) {
-  if (bytes <= 48 * 1024) return LMM_OK;
-  static std::mutex mu;
-  static std::vector<std::pair<const void*, int>> done;
-  int dev = 0;
-  int st = check_cuda(cudaGetDevice(&dev), "ls_date_kernel: cudaGetDevice");
-  if (st) return st;
-  std::lock_guard<std::mutex> lock(mu);
-  for (const auto& d : done)
-    if (d.first == (const void*)kern && d.second == dev) return LMM_OK;
-  st = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)bytes),
-                  "ls_date_kernel: shared memory attribute");
-  if (st) return st;
-  done.emplace_back((const void*)kern, dev);
-  return LMM_OK;
-}
-
 // Launch the date kernel instantiated for the smallest slot count KR >=
 // nbasis + 1 (rows split over warp pairs above 11 slots).
 int launch_date(const LSDateParams& P_in, int grid, const float* vars,
@@ -1067,7 +1044,8 @@ int launch_date(const LSDateParams& P_in, int grid, const float* vars,
 #define LMM_LS_DATE(KR, NS, KIND)                                                    \
   do {                                                                               \
     constexpr size_t sb = ls_stage_bytes<KR, NS, false>();                           \
-    const int at = ls_stage_attr(ls_date_kernel<KR, NS, KIND, false>, sb);           \
+    const int at = allow_smem((const void*)ls_date_kernel<KR, NS, KIND, false>, sb,  \
+                              "ls_date_kernel: shared memory attribute");            \
     if (at) return at;                                                               \
     ls_date_kernel<KR, NS, KIND, false><<<grid, LsThreads<KR>::value, sb, s>>>(      \
         P, vars, means, sds, cf, ex, num, beta, y, part, counter, gram, status, sums_out); \
@@ -1075,7 +1053,8 @@ int launch_date(const LSDateParams& P_in, int grid, const float* vars,
 #define LMM_LS_DATE_MASKED(KR, NS, KIND)                                             \
   do {                                                                               \
     constexpr size_t sb = ls_stage_bytes<KR, NS, true>();                            \
-    const int at = ls_stage_attr(ls_date_kernel<KR, NS, KIND, true>, sb);            \
+    const int at = allow_smem((const void*)ls_date_kernel<KR, NS, KIND, true>, sb,   \
+                              "ls_date_kernel: shared memory attribute");            \
     if (at) return at;                                                               \
     ls_date_kernel<KR, NS, KIND, true><<<grid, LsThreads<KR>::value, sb, s>>>(       \
         P, vars, means, sds, cf, ex, num, beta, y, part, counter, gram, status, sums_out); \
@@ -1143,7 +1122,7 @@ int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const 
     R.known[e] = kind != kBasisGeneric && ls_basis_kind(R.date[e]) == kind;
   auto go = [&](auto kern, int pairs, size_t stage, int threads) -> int {
     double* part1 = part + (size_t)nblk * pairs;
-    int st = ls_stage_attr(kern, stage);
+    int st = allow_smem((const void*)kern, stage, "ls_run_kernel: shared memory attribute");
     if (st) return st;
     const int grid = std::min(div_up(R.paths, threads), nblk);
     void* args[] = {&R, &vars, &means, &sds, &cf, &ex, &num, &beta, &y, &part, &part1,

@@ -348,9 +348,7 @@ int path_gram_launch(int m, int n, int paths, const float* X, int ldx,
   const int nb = path_gram_blocks(paths);
   const size_t smem = path_gram_smem(n, same);
   auto go = [&](auto kern) -> int {
-    int st = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem),
-                        "lmm_path_gram: smem attribute");
+    int st = allow_smem((const void*)kern, smem, "lmm_path_gram: smem attribute");
     if (st) return st;
     kern<<<nb, kThreads, smem, s>>>(m, n, paths, X, ldx, Y, ldy, same, part, status);
     return check_launch("path_gram_kernel");

@@ -457,9 +457,7 @@ int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
   const size_t smem = pairs ? pair_smem_bytes(rows, v.F, rows - tmem_rows)
                                    : fused_smem_bytes(rows, v.F, block);
   auto attr = [&](auto kern) -> int {
-    return check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem),
-                      "fused: smem attribute");
+    return allow_smem((const void*)kern, smem, "fused: smem attribute");
   };
   return dispatch_factors(v.F, [&](auto ft) -> int {
     constexpr int FT = decltype(ft)::value;
@@ -585,10 +583,7 @@ int launch_variates(const Validated& v, const lmm_model* m, int P, uint32_t off,
   VarPlan vp;
   make_var_plan(plan, &vp);
   const size_t smem = variates_smem_bytes(vp);
-  TRY(check_cuda(cudaFuncSetAttribute(variates_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem),
-                 "variates: smem attribute"));
+  TRY(allow_smem((const void*)variates_kernel, smem, "variates: smem attribute"));
   // several tiles per CTA, so that the Sobol tables and the bridge plan are
   // built once for them, while the grid still holds every SM's CTAs (eight or
   // so) several times over
@@ -710,9 +705,7 @@ int launch_tensor(const Validated& v, int P, const float* Z, const lmm_model* m,
   tc_b_image_kernel<<<dim3(G.NB, v.n), G.KT, 0, s>>>(v.n, v.F, m->d_A, img);
   TRY(check_launch("tc_b_image_kernel"));
   const size_t smem = tc_evolve_smem(v.n);
-  TRY(check_cuda(cudaFuncSetAttribute(tc_evolve_kernel<MODE>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                 "tensor evolution: smem attribute"));
+  TRY(allow_smem((const void*)tc_evolve_kernel<MODE>, smem, "tensor evolution: smem attribute"));
   tc_evolve_kernel<MODE><<<div_up(P, tc::kThreads), tc::kThreads, smem, s>>>(
       P, Z, v.F, img, m->d_fixed_drifts, v.mc, v.pc, v.rc, rule, total, col, vars,
       ex, cf, num, payoff, errors);
@@ -1100,9 +1093,7 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
   };
   auto resident = [&](int* ctas) -> int {
     return dispatch_reverse([&](auto kern) -> int {
-      TRY(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)smem_rev),
-                     "greeks: reverse smem"));
+      TRY(allow_smem((const void*)kern, smem_rev, "greeks: reverse smem"));
       int per_sm = 0;
       TRY(check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRevThreads,
                                                                    smem_rev),
@@ -1146,9 +1137,7 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
     constexpr int FT = decltype(ft)::value;
     const void* kern = pairs ? (const void*)greeks_segment_pairs_kernel<FT>
                              : (const void*)greeks_segment_kernel<FT>;
-    return check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem_seg),
-                      "greeks: segment smem");
+    return allow_smem(kern, smem_seg, "greeks: segment smem");
   }));
   auto seg_range = [&](int cp, int& s0, int& s1) {
     s0 = cp * k;
@@ -1425,9 +1414,7 @@ extern "C" int lmm_andersen_broadie(const lmm_model* model, const lmm_product* p
   const unsigned grid = (unsigned)((size_t)(E - 1) * (((size_t)K * chunks + 1) / 2));
   TRY(dispatch_factors(v.F, [&](auto ft) -> int {
     auto kern = ab_inner_kernel<decltype(ft)::value>;
-    TRY(check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem),
-                   "ab_inner: smem attribute"));
+    TRY(allow_smem((const void*)kern, smem, "ab_inner: smem attribute"));
     kern<<<grid, kPairThreads, smem, s>>>(a, model->d_A, model->d_fixed_drifts, v.mc, v.pc, v.rc,
                                           view, b.ckpt, b.ckptN, b.part, n - tmem_rows);
     return check_launch("ab_inner_kernel");
