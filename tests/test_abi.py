@@ -304,3 +304,32 @@ def test_segmented_price_rejects_bad_inputs():
     model3, prod3, keep3 = _mini_model_product(kind=2)  # European strip: never stops
     assert LIB.lmm_fused_price_workspace_bytes(ctypes.addressof(model3),
                                                ctypes.addressof(prod3), 1000) == 256
+
+
+@pytest.mark.parametrize("n,F", [(40, 5), (20, 10), (20, 3), (80, 10), (30, 16)])
+def test_workspaces_serve_fewer_paths(n, F):
+    """A workspace sized for P paths holds any smaller batch: the sizes do not
+    fall where the number of paths changes the kernel (two paths per thread
+    from 100,000 or 160,000 paths and n F P = 2^23)."""
+    from useful_code_b200.pricer import LmmModel, LmmProduct
+
+    taus = np.full(n, 0.5, np.float32)
+    disp = np.zeros(n, np.float32)
+    f0 = np.full(n, 0.05, np.float32)
+    model = LmmModel(n, F, p(taus), p(disp), p(f0), FAKE, FAKE, FAKE, None, 0, 10.0)
+    ex = np.arange(n, dtype=np.int32)
+    nv = np.full(n, 3, np.int32)
+    nv[-1] = 1
+    mono, nb = mk.basis_tables("quadratic", nv)
+    prod = LmmProduct(0, 0.05, 0.05, 1.0, n, p(ex), p(nv), p(mono), p(nb), 1)
+    m, pr = ctypes.addressof(model), ctypes.addressof(prod)
+    sizes = {
+        "price": lambda q: LIB.lmm_fused_price_workspace_bytes(m, pr, q),
+        "pipeline": lambda q: LIB.lmm_pipeline_workspace_bytes(m, pr, q, 1),
+        "greeks": lambda q: LIB.lmm_greeks_workspace_bytes(m, pr, q, 8),
+    }
+    edge = -(-(1 << 23) // (n * F))
+    for name, size in sizes.items():
+        for around in (128, 256, 56000, 100000, 160000, edge):
+            got = [size(q) for q in range(around - 20, around + 21)]
+            assert got[0] > 0 and got == sorted(got), (name, around)

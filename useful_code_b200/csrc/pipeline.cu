@@ -494,11 +494,15 @@ struct SegBufs {
   int blocks, cap;
 };
 
+// The buffers' sizes do not depend on which kernel runs the chain: survivors
+// rounded up to the larger CTA, counts for the smaller one, so that a
+// workspace for P paths serves every smaller number of paths too.
 SegBufs carve_seg(Carver& c, const Validated& v, int P) {
   SegBufs b;
-  const int block = evolve_block(v, P, true);
-  b.blocks = div_up(P, block);
-  b.cap = b.blocks * block;
+  static_assert(kPairBlock % kFusedBlock == 0, "CTAs of either kernel fill the survivors");
+  b.blocks = div_up(P, evolve_block(v, P, true));
+  b.cap = div_up(P, kPairBlock) * kPairBlock;
+  const size_t counts = (size_t)(b.cap / kFusedBlock);
   const size_t cap = (size_t)b.cap;
   for (SegState& st : b.st) {
     st.rates = c.take<float>((size_t)v.n * cap);
@@ -509,8 +513,8 @@ SegBufs carve_seg(Carver& c, const Validated& v, int P) {
     st.payoff = c.take<double>(cap);
     st.path = c.take<int>(cap);
   }
-  b.count = c.take<int>((size_t)b.blocks);
-  b.prefix = c.take<int>((size_t)b.blocks + 1);
+  b.count = c.take<int>(counts);
+  b.prefix = c.take<int>(counts + 1);
   return b;
 }
 
