@@ -411,7 +411,12 @@ int lmm_step_to_exercise_indices(const int* h_gen_indices, int n_gen,
  * (FP64), optional d_gram[E][16][17] (normalised Gram | target column),
  * d_status (bit 1: zero Gram, 2: Cholesky failed, 4: jitter used, 32: a
  * bounded wait between the launch's CTAs ran out) and
- * d_price = mean_p y_p / N_0(p).  Workspace: lmm_ls_workspace_bytes(). */
+ * d_price = mean_p y_p / N_0(p).  Workspace: lmm_ls_workspace_bytes().
+ * With at most 10 functions per date the backward loop is one cooperative
+ * launch of at most one CTA per SM; on a stream that owns too few SMs for it
+ * (a green context's), and with more functions, it is one launch per date,
+ * with the same results to the last bit.  Two regressions on two streams may
+ * therefore run one after the other.  The call can be captured in a graph. */
 size_t lmm_ls_workspace_bytes(int paths, int n_exercise);
 int lmm_ls_regress(int n_exercise, int paths, const float* d_vars,
                    const int* h_nvars, const uint8_t* h_monomials,
@@ -551,8 +556,12 @@ typedef struct lmm_ls_rule {
  * half-width search stopped after 512 count evaluations, where the
  * reference's search does not end, e.g. more than the upper target of net
  * values exactly zero; 16: a search needed more than its device passes; 32:
- * a bounded wait between the launch's CTAs ran out) and d_price = mean_p y_p / N_0(p).  Everything stays on the device: no host
- * synchronisation inside, so the call can be captured in a graph.
+ * a bounded wait between the launch's CTAs ran out) and
+ * d_price = mean_p y_p / N_0(p).  Everything stays on the device: no host
+ * synchronisation inside, so the call can be captured in a graph.  The path
+ * selections are cooperative launches of at most one CTA per SM of the stream
+ * (of its green context, where it has one; their FP64 sums over CTAs then
+ * have fewer terms).
  * Workspace: lmm_ls_nested_workspace_bytes(). */
 size_t lmm_ls_nested_workspace_bytes(int paths, int n_exercise);
 int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_vars,

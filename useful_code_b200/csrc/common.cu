@@ -1,6 +1,8 @@
 // common.cu — status/error plumbing shared by every C-ABI entry point.
 #include "lmm_common.cuh"
 
+#include <cuda.h>
+
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -55,6 +57,35 @@ int sm_count() {
     cached[dev] = n;
   }
   return cached[dev];
+}
+
+namespace {
+template <class Fn>
+Fn driver_fn(const char* name) {
+  void* f = nullptr;
+  cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+  if (cudaGetDriverEntryPointByVersion(name, &f, 12040, cudaEnableDefault, &found) !=
+          cudaSuccess ||
+      found != cudaDriverEntryPointSuccess)
+    return nullptr;
+  return reinterpret_cast<Fn>(f);
+}
+}  // namespace
+
+int stream_sm_count(cudaStream_t s) {
+  static const auto green_of =
+      driver_fn<CUresult (*)(CUstream, CUgreenCtx*)>("cuStreamGetGreenCtx");
+  static const auto resource_of =
+      driver_fn<CUresult (*)(CUgreenCtx, CUdevResource*, CUdevResourceType)>(
+          "cuGreenCtxGetDevResource");
+  const int all = sm_count();
+  CUgreenCtx green = nullptr;
+  CUdevResource res;
+  if (!green_of || !resource_of || green_of((CUstream)s, &green) != CUDA_SUCCESS || !green ||
+      resource_of(green, &res, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+    return all;
+  const int own = (int)res.sm.smCount;
+  return own > 0 && own < all ? own : all;
 }
 
 // A kernel's limit is one value for all threads of the process.  One made to

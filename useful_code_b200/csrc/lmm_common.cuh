@@ -40,6 +40,11 @@ inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+// Number of SMs that launches on `s` may use: the device's, or the part of
+// them that the stream's green context owns.  A cooperative launch has to fit
+// them with all of its CTAs at once.
+int stream_sm_count(cudaStream_t s);
+
 // Grid size for a grid-stride kernel: enough CTAs to fill every SM `per_sm`
 // times, but never more than the work needs.
 inline int grid_for(long long work_items, int block, int per_sm = 8) {

@@ -1101,7 +1101,9 @@ int launch_date(const LSDateParams& P_in, int grid, const float* vars,
 
 // The whole backward loop (ls_run_kernel), instantiated for the most slots
 // of any date and for the table that most dates share; -1 (nothing launched)
-// for tables of more than 11 slots.  `part` holds nblk x kLsMaxPairs doubles,
+// for tables of more than 11 slots, and on a stream that owns too few SMs to
+// hold all CTAs at once (a green context's): the loop of one launch per date
+// waits for nobody and gives the same bits.  `part` holds nblk x kLsMaxPairs doubles,
 // room for two buffers of 66.
 int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const float* sds,
                const float* cf, const float* ex, const float* num, double* beta, float* y,
@@ -1122,9 +1124,10 @@ int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const 
     R.known[e] = kind != kBasisGeneric && ls_basis_kind(R.date[e]) == kind;
   auto go = [&](auto kern, int pairs, size_t stage, int threads) -> int {
     double* part1 = part + (size_t)nblk * pairs;
+    const int grid = std::min(div_up(R.paths, threads), nblk);
+    if (grid > stream_sm_count(s)) return -1;
     int st = allow_smem((const void*)kern, stage, "ls_run_kernel: shared memory attribute");
     if (st) return st;
-    const int grid = std::min(div_up(R.paths, threads), nblk);
     void* args[] = {&R, &vars, &means, &sds, &cf, &ex, &num, &beta, &y, &part, &part1,
                     &counter, &gram, &status};
     st = check_cuda(cudaLaunchCooperativeKernel((const void*)kern, dim3(grid), dim3(threads),
@@ -1209,7 +1212,7 @@ extern "C" int lmm_ls_regress(int n_exercise, int paths, const float* d_vars,
   st = launch_run(run, nblk, d_vars, means, sds, d_cf, d_ex, d_num, d_beta, y, part, counter,
                   d_gram, d_status, s);
   if (st > 0) return st;
-  // tables of more than 11 slots: one launch per date
+  // otherwise one launch per date
   for (int e = n_exercise - 1; st < 0 && e >= 0; --e) {
     LSDateParams P;
     memset(&P, 0, sizeof(P));

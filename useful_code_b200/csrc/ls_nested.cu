@@ -728,7 +728,8 @@ extern "C" int lmm_ls_regress_nested(int n_exercise, int paths, const float* d_v
   }
   const int nblk = ls_gram_blocks();
   const int grid_path = grid_for(paths, kNestThreads, 4);
-  const int grid_sel = std::min(div_up(paths, kSelThreads), nblk);
+  // cooperative launches: no more CTAs than the stream's SMs hold at once
+  const int grid_sel = std::min(div_up(paths, kSelThreads), std::min(nblk, stream_sm_count(s)));
   int launches = 0;
   const LsRuleView rule{D, d_beta, means, sds, D > 1 ? d_cuts : nullptr, nullptr};
   for (int e = n_exercise - 1; e >= 0; --e) {
