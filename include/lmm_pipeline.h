@@ -264,7 +264,10 @@ int lmm_ls_apply_rule_nested(int n_exercise, int paths, const float* d_vars,
  *                                        A_s[r] -> k_r A_s[r] of every step
  *   d_exercise_step [paths] (or NULL)    each path's exercise step under the
  *                                        rule (rates = never), int32
- * paths must be a multiple of 4.  Vegas to other volatility parameters
+ * paths must be a multiple of 4.  The workspace grows with the paths; besides, it holds the
+ * reverse sweep's partial sums: two buffers of min(checkpoint_every, 8) steps of
+ * up to 4 CTAs per SM, rates (factors + 2) FP64 values each (73 MB at 80 rates
+ * and 10 factors on 148 SMs).  Vegas to other volatility parameters
  * follow by the chain rule through the host pseudo-root construction
  * (lmm_abcd_vegas in lmm_c.h).  The call is ordered on `stream` like every
  * other entry point; inside it, the reverse sweep and the recompute of the

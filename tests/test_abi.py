@@ -333,3 +333,28 @@ def test_workspaces_serve_fewer_paths(n, F):
         for around in (128, 256, 56000, 100000, 160000, edge):
             got = [size(q) for q in range(around - 20, around + 21)]
             assert got[0] > 0 and got == sorted(got), (name, around)
+
+
+def test_greeks_partials_are_bounded():
+    """Beyond four CTAs of 128 paths per SM the reverse sweep's partial sums
+    stop growing: the workspace for 8-step segments, less the one for 4-step
+    segments, is then a multiple of the paths plus four steps of partials of
+    rates (factors + 2) FP64 sums for 4 x 148 CTAs, held twice."""
+    from useful_code_b200.pricer import LmmModel, LmmProduct
+
+    n, F = 80, 10
+    a = [np.full(n, x, np.float32) for x in (0.5, 0.0, 0.05)]
+    model = LmmModel(n, F, p(a[0]), p(a[1]), p(a[2]), FAKE, FAKE, FAKE, None, 0, 10.0)
+    ex, nv = np.arange(n, dtype=np.int32), np.full(n, 3, np.int32)
+    nv[-1] = 1
+    mono, nb = mk.basis_tables("quadratic", nv)
+    prod = LmmProduct(0, 0.05, 0.05, 1.0, n, p(ex), p(nv), p(mono), p(nb), 1)
+
+    def more(paths):  # of 8-step segments over 4-step ones
+        size = [LIB.lmm_greeks_workspace_bytes(ctypes.addressof(model), ctypes.addressof(prod),
+                                               paths, k) for k in (4, 8)]
+        return size[1] - size[0]
+
+    # whole tiles: everything else is exactly proportional to the paths
+    fixed = 2 * more(1 << 20) - more(1 << 21)
+    assert fixed == 2 * 4 * (4 * 148) * n * (F + 2) * 8

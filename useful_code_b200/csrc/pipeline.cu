@@ -624,9 +624,10 @@ size_t greeks_seg_floats(size_t n, size_t P, int k) {
   return (size_t)k * n * ((P + kRevThreads - 1) / kRevThreads) * kSegRow;
 }
 
-// Upper bound on the CTAs of the reverse kernel (sizes the partials).
+// Upper bound on the CTAs of the reverse kernel (sizes the partials, and bounds
+// the launch): its register counts, 110 to 224, let an SM hold four at most.
 int greeks_reverse_grid(int P) {
-  return std::min(div_up(P, kRevThreads), 6 * sm_count());
+  return std::min(div_up(P, kRevThreads), 4 * sm_count());
 }
 
 GreeksBufs carve_greeks(Carver& c, const Validated& v, size_t P, int k) {
