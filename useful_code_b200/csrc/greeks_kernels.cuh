@@ -612,17 +612,20 @@ __host__ __device__ constexpr int rev_stage_floats(int FM) { return 32 * rev_sta
 // 3.1 (2^20 paths: 45.0 -> 39.0).  Without the prefetch the last would be
 // about 10% slower; 240 registers and two CTAs per SM, or one path per thread
 // and four, gave 12.2 at 2^18 with the five products.
-template <int FT, int NPATH_>
+// Two paths per thread need the registers of 10 factors or fewer; more factors
+// (and the generic form) always run one, in 222 and 224 registers.
+template <int FT>
 struct RevShape {
-  // paths per thread; one where all tiles are resident at once (small
-  // launches are bound by a warp's chain, which two paths lengthen)
-  static constexpr int NPATH = (FT > 0 && FT <= 10) ? NPATH_ : 1;
-  static constexpr int MINB = NPATH == 1 ? ((FT > 0 && FT <= 10) ? 4 : 1)
-                                         : FT <= 5 ? 4 : 3;
+  static constexpr int kMost = (FT > 0 && FT <= 10) ? 2 : 1;  // paths per thread
+  static constexpr int min_ctas(int npath) {
+    return kMost == 1 ? 1 : (npath == 1 || FT <= 5) ? 4 : 3;
+  }
 };
 
-template <int FT, int NPATH_>
-__global__ void __launch_bounds__(kRevThreads, RevShape<FT, NPATH_>::MINB)
+// NPATH 1 where all tiles are resident at once: small launches are bound by a
+// warp's chain, which two paths lengthen.
+template <int FT, int NPATH>
+__global__ void __launch_bounds__(kRevThreads, RevShape<FT>::min_ctas(NPATH))
     greeks_reverse_kernel(int paths, int s_hi, int s_lo, const int* __restrict__ cnt, int chunks,
                           const float* __restrict__ A,
                           const __grid_constant__ ModelConst mc,
@@ -636,7 +639,6 @@ __global__ void __launch_bounds__(kRevThreads, RevShape<FT, NPATH_>::MINB)
   constexpr int NC = rev_stage_cols(FM);
   constexpr int NS = FM + 2;        // summed columns: FM factors, the adjoint, L
   constexpr int LAMC = 2 * NP;      // stage column of the rate adjoint
-  constexpr int NPATH = RevShape<FT, NPATH_>::NPATH;
   constexpr int kUnits = kSortChunk / (T * NPATH);  // per chunk
   const int F = FT > 0 ? FT : mc.F;
   const int n = mc.n;

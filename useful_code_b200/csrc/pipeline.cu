@@ -1093,7 +1093,8 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
   auto dispatch_reverse = [&](auto&& go) -> int {
     return dispatch_factors(F, [&](auto ft) -> int {
       constexpr int FT = decltype(ft)::value;
-      return rev_one ? go(greeks_reverse_kernel<FT, 1>) : go(greeks_reverse_kernel<FT, 2>);
+      return rev_one ? go(greeks_reverse_kernel<FT, 1>)
+                     : go(greeks_reverse_kernel<FT, RevShape<FT>::kMost>);
     });
   };
   auto resident = [&](int* ctas) -> int {
