@@ -160,3 +160,33 @@ def test_bounds_bracket_the_price(swaption_rules):
     assert r.gap < 0.05 * price
     print(f"AB mini swaption: lower {r.lower:.6f} +- {r.lower_se:.6f}, gap {r.gap:.6f} "
           f"+- {r.gap_se:.6f}, second pass {price:.6f}")
+
+
+@pytest.mark.parametrize("model,n,F,K", [("c3", 80, 10, 5), ("c2", 61, 5, 7), ("c5", 120, 15, 3),
+                                         ("c3", 75, 16, 5), ("c2", 59, 3, 1)])
+def test_inner_estimates_of_large_models(cuda, model, n, F, K):
+    """Every compiled factor count and the generic one, at rate counts whose
+    last log-rates lie in tensor memory (from 53 rates of 3 or 5 factors and 67
+    of more), with an odd number of 128-path units per date, so that
+    one warp pair of the last CTA is idle: continuation estimates against the
+    oracle on the device's outer states and the same normals.  A flipped inner
+    decision moves an estimate by at most an exercise value / 128."""
+    from dataclasses import replace
+
+    from useful_code_b200.pricer import Pipeline
+
+    cfg = mk.make_config(model)
+    m = mk.build_market(replace(cfg, n=n, F=F, f0=np.resize(cfg.f0, n).astype(np.float32),
+                                product="swaption"))
+    pipe = Pipeline(m)
+    rule = pipe.regress(pipe.first_pass(1 << 14, 0))
+    inner, seed = 128, 11223344
+    r = pipe.andersen_broadie(rule, K, 1 << 15, inner, seed=seed, keep=True)
+    Qg = r.Q.cpu().numpy()
+    E = Qg.shape[0]
+    Qo, _ = _oracle_ab_inner(m, rule, r.ckpt.cpu().numpy(), r.ckptN.cpu().numpy(), K, inner,
+                             seed, 0, E)
+    diff = np.abs(Qg - Qo)
+    assert np.mean(diff < 1e-6) > 0.97, np.sort(diff.ravel())[-10:]
+    assert diff.max() < 4e-3
+    assert np.abs(Qg[-1]).max() == 0.0

@@ -268,14 +268,16 @@ def test_generic_factor_counts(cuda, F):
     assert abs(float(np.sum(g.abar * D)) - fdv) < 2e-4 * abs(fdv) + 1e-9
 
 
-@pytest.mark.parametrize("P", [12, 4100, 8324])
+@pytest.mark.parametrize("P", [12, 4100, 8324, 77956])
 def test_ordered_sweep_ragged_counts(cuda, P):
     """The reverse sweep takes the paths in chunks of 4096 ordered by their
-    last step with work, two tiles of 128 positions per thread: path counts
-    that leave a short last chunk and a short last tile (12 paths: one
-    partial tile; 4100: a chunk of 4 paths; 8324: a chunk of 132, a tile of
-    4) against the FP64 frozen-exercise differences, and two calls in a row
-    bit-identical (the order and every sum are fixed)."""
+    last step with work, in tiles of 128 positions; one position per thread
+    while all tiles are resident, two tiles per thread above (77956 paths: 610
+    tiles, 592 places).  Path counts that leave a short last chunk and a short
+    last tile (12 paths: one partial tile; 4100: a chunk of 4 paths; 8324: a
+    chunk of 132, a tile of 4; 77956: a chunk of 132) against the FP64
+    frozen-exercise differences, and two calls in a row bit-identical (the
+    order and every sum are fixed)."""
     m, pipe, rule, _ = setup("swaption")
     g = pipe.greeks(P, 4096, rule, checkpoint_every=4)
     g2 = pipe.greeks(P, 4096, rule, checkpoint_every=4)
@@ -293,9 +295,8 @@ def test_ordered_sweep_ragged_counts(cuda, P):
 
 @pytest.mark.parametrize("n,F", [(12, 5), (16, 10), (16, 15)])
 def test_compiled_factor_counts(cuda, n, F):
-    """The factor counts with kernels of their own (5: six CTAs per SM, two
-    paths per thread; 10: the bench's shape; 15: one path per thread):
-    deltas and a random dV/dA direction against the FP64 frozen-exercise
+    """The factor counts with kernels of their own, in the form for few paths
+    (one per thread; more paths: test_pairs_gpu.py): deltas and a random dV/dA direction against the FP64 frozen-exercise
     differences."""
     m, pipe, rule, P = setup("swaption", n=n, F=F, f0=np.linspace(0.04, 0.06, n).astype(np.float32))
     g = pipe.greeks(P, P, rule, checkpoint_every=5)

@@ -34,7 +34,8 @@ def pipeline(model, n, F, **kw):
 # every compiled factor count and the generic one, odd path counts
 SHAPES = [("c3", 80, 10, 100003), ("c2", 40, 5, 160001), ("c5", 120, 15, 100511),
           ("c2", 37, 5, 163333), ("c3", 128, 10, 100481), ("c5", 61, 16, 100737),
-          ("c3", 50, 4, 165601), ("c2", 47, 3, 160961), ("c3", 19, 16, 104001)]
+          ("c3", 50, 4, 165601), ("c2", 47, 3, 160961), ("c3", 19, 16, 104001),
+          ("c2", 64, 3, 160233), ("c2", 57, 5, 161003), ("c5", 70, 16, 100111)]
 
 
 @pytest.mark.parametrize("model,n,F,P", SHAPES)
@@ -195,3 +196,56 @@ def test_threads_price_at_once(cuda):
     for t in threads:
         t.join()
     assert not errors
+
+
+# the reverse sweep takes two paths per thread from 75,777 paths (593 tiles, up
+# to 10 factors) and the recompute from 56,000 (n F P >= 2^23); 15 factors and
+# the generic form keep one in the reverse sweep
+@pytest.mark.parametrize("model,n,F,P,product", [
+    ("c3", 80, 10, 100004, "swaption"), ("c2", 40, 5, 81932, "cancellable"),
+    ("c3", 24, 10, 77828, "bermudan_cap"), ("c1", 28, 5, 75780, "european"),
+    ("c2", 37, 3, 82052, "swaption"), ("c5", 30, 15, 60004, "swaption"),
+    ("c3", 21, 16, 57004, "cancellable")])
+def test_greeks_batches(cuda, model, n, F, P, product):
+    """Greeks of P paths are the path-weighted sums of its batches' Greeks.
+    Per path every value is the same; a thread's and a warp's FP32 sums join
+    64 paths of the batch's instead of 32, and each of the up to 63 additions
+    rounds its partial sum by 2^-24 at most.  Rows of dV/dA cancel little, so
+    the 2-norm differs by less than 63 * 2^-24 = 3.8e-6 of the result."""
+    pipe = pipeline(model, n, F, product=product)
+    euro = product == "european"
+    rule = None if euro else pipe.regress(pipe.first_pass(8192, 0))
+    whole = pipe.greeks(P, 99999, rule)
+    price, delta, abar, vega, ex = 0.0, 0.0, 0.0, 0.0, []
+    for lo in range(0, P, BATCH):
+        size = min(BATCH, P - lo)
+        g = pipe.greeks(size, 99999 + lo, rule)
+        w = size / P
+        price += w * g.price
+        delta, abar, vega = delta + w * g.delta, abar + w * g.abar, vega + w * g.vega_rate
+        ex.append(g.exercise_step)
+    assert np.array_equal(whole.exercise_step, np.concatenate(ex))
+    assert abs(whole.price - price) < 1e-12 * abs(price)
+    for name, ref in (("delta", delta), ("abar", abar), ("vega_rate", vega)):
+        got = getattr(whole, name)
+        assert np.linalg.norm(got - ref) < 3.8e-6 * np.linalg.norm(ref), name
+
+
+@pytest.mark.parametrize("model,n,F,K", [("c3", 16, 10, 56007), ("c2", 30, 5, 56004),
+                                         ("c3", 50, 3, 56001), ("c5", 28, 15, 20485),
+                                         ("c3", 27, 16, 20483)])
+def test_bound_outer_paths(cuda, model, n, F, K):
+    """Outer paths of the Andersen-Broadie bound, two per thread, against a
+    call with fewer, one per thread: states, decisions, exercise values and the
+    continuation estimates from them (inner paths are counted by the outer
+    path's number), bit for bit."""
+    pipe = pipeline(model, n, F, product="swaption")
+    rule = pipe.regress(pipe.first_pass(8192, 0))
+    whole = pipe.andersen_broadie(rule, K, 4321, 128, keep=True)
+    few = 501
+    part = pipe.andersen_broadie(rule, few, 4321, 128, keep=True)
+    for name in ("ckpt", "ckptN", "X", "Z", "Q"):
+        assert torch.equal(getattr(whole, name)[..., :few], getattr(part, name)), name
+    tail = pipe.andersen_broadie(rule, 257, 4321 + K - 257, 128, keep=True)
+    for name in ("ckpt", "ckptN", "X", "Z"):
+        assert torch.equal(getattr(whole, name)[..., K - 257:], getattr(tail, name)), name
