@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
+#include <vector>
 
 using namespace lmm;
 
@@ -1024,6 +1025,25 @@ size_t ls_workspace_bytes(int paths, int n_ex) {
   return y + part + cnt + mom + red + 256;
 }
 
+// allow_smem once per kernel and device: a date launch always asks for the
+// same, and the sharded protocol's host work shows every driver call (1.2 us
+// of 32 us a date).
+template <class Kern>
+int ls_stage_attr(Kern kern, size_t bytes) {
+  static std::mutex mu;
+  static std::vector<std::pair<const void*, int>> done;
+  int dev = 0;
+  int st = check_cuda(cudaGetDevice(&dev), "ls_date_kernel: cudaGetDevice");
+  if (st) return st;
+  std::lock_guard<std::mutex> lock(mu);
+  for (const auto& d : done)
+    if (d.first == (const void*)kern && d.second == dev) return LMM_OK;
+  st = allow_smem((const void*)kern, bytes, "ls_date_kernel: shared memory attribute");
+  if (st) return st;
+  done.emplace_back((const void*)kern, dev);
+  return LMM_OK;
+}
+
 // Launch the date kernel instantiated for the smallest slot count KR >=
 // nbasis + 1 (rows split over warp pairs above 11 slots).
 int launch_date(const LSDateParams& P_in, int grid, const float* vars,
@@ -1044,8 +1064,7 @@ int launch_date(const LSDateParams& P_in, int grid, const float* vars,
 #define LMM_LS_DATE(KR, NS, KIND)                                                    \
   do {                                                                               \
     constexpr size_t sb = ls_stage_bytes<KR, NS, false>();                           \
-    const int at = allow_smem((const void*)ls_date_kernel<KR, NS, KIND, false>, sb,  \
-                              "ls_date_kernel: shared memory attribute");            \
+    const int at = ls_stage_attr(ls_date_kernel<KR, NS, KIND, false>, sb);           \
     if (at) return at;                                                               \
     ls_date_kernel<KR, NS, KIND, false><<<grid, LsThreads<KR>::value, sb, s>>>(      \
         P, vars, means, sds, cf, ex, num, beta, y, part, counter, gram, status, sums_out); \
@@ -1053,8 +1072,7 @@ int launch_date(const LSDateParams& P_in, int grid, const float* vars,
 #define LMM_LS_DATE_MASKED(KR, NS, KIND)                                             \
   do {                                                                               \
     constexpr size_t sb = ls_stage_bytes<KR, NS, true>();                            \
-    const int at = allow_smem((const void*)ls_date_kernel<KR, NS, KIND, true>, sb,   \
-                              "ls_date_kernel: shared memory attribute");            \
+    const int at = ls_stage_attr(ls_date_kernel<KR, NS, KIND, true>, sb);            \
     if (at) return at;                                                               \
     ls_date_kernel<KR, NS, KIND, true><<<grid, LsThreads<KR>::value, sb, s>>>(       \
         P, vars, means, sds, cf, ex, num, beta, y, part, counter, gram, status, sums_out); \
@@ -1126,7 +1144,7 @@ int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const 
     double* part1 = part + (size_t)nblk * pairs;
     const int grid = std::min(div_up(R.paths, threads), nblk);
     if (grid > stream_sm_count(s)) return -1;
-    int st = allow_smem((const void*)kern, stage, "ls_run_kernel: shared memory attribute");
+    int st = ls_stage_attr(kern, stage);
     if (st) return st;
     void* args[] = {&R, &vars, &means, &sds, &cf, &ex, &num, &beta, &y, &part, &part1,
                     &counter, &gram, &status};
