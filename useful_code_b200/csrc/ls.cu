@@ -646,7 +646,12 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
 //
 // For tables of at most 11 slots, whose rows one warp holds.  80 dates, 10
 // functions: 2.85 -> 2.19 ms at 2^20 paths, 1.97 -> 1.33 at 2^18; 40 dates, 6
-// functions: 0.70 -> 0.41 ms at 2^16, 0.62 -> 0.39 at 4,099.  Larger tables
+// functions: 0.70 -> 0.41 ms at 2^16, 0.62 -> 0.39 at 4,099.  VEC16: rows
+// copied in 16-byte chunks (aligned rows, a path count that is a multiple of
+// four), else value by value, from row pointers in shared memory: found anew
+// for every copy they cost 3.92 ms at 1,000,001 paths against 3.20 with one
+// launch per date, so 2.55; both copies in one kernel made aligned
+// regressions with generic tables 15% slower.  Larger tables
 // keep one launch per date: with their rows split over warp pairs the loop
 // gained less (120 dates, 12 functions, 2.65 against 3.0 ms at 150,001 paths),
 // and there the compiler contracts other products into the sums than in
@@ -654,14 +659,14 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
 // coefficient.
 // ---------------------------------------------------------------------------
 struct LSRun {
-  int n_ex, paths, vec16;
+  int n_ex, paths;
   unsigned char known[kMaxSteps];  // the date's table is the launch's KIND
   LSDate date[kMaxSteps];
 };
 
 constexpr int kLsWait = 32;  // status: a wait of the grid ran out
 
-template <int KR, int KIND>
+template <int KR, int KIND, bool VEC16>
 __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
     ls_run_kernel(const __grid_constant__ LSRun R, const float* __restrict__ vars,
                   const float* __restrict__ means, const float* __restrict__ sds,
@@ -690,7 +695,9 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
   const int r0 = lane >> 3, c4 = (lane & 7) * 4;
   float* const wstage = ls_stage + warp * 32;
   const int w0 = blockIdx.x * T + warp * 32, stride = gridDim.x * T;
-  // input row i of date e's loop (null: not read)
+  // input rows of the date in src_s[date & 1] (null: not read), those of the
+  // next date written while the loop still reads this one's
+  __shared__ const float* src_s[2][kLsInputs];
   auto row_ptr = [&](int e, int i) -> const float* {
     const size_t cur = (size_t)e * paths, nxt = cur + paths;
     if (i < kInCf)
@@ -712,7 +719,7 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
   // aligned, else each lane its own path's values)
   auto issue = [&](int e, int it, int qw) {
     float* dst = wstage + (it & (kLsStages - 1)) * kLsInputs * T;
-    if (R.vec16) {
+    if (VEC16) {
       const int qb = qw + c4;
       if (qb < paths) {
         if (rp0) cp_async16(dst + r0 * T + c4, rp0 + qb);
@@ -720,20 +727,16 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
         if (rp2) cp_async16(dst + (r0 + 8) * T + c4, rp2 + qb);
       }
     } else if (qw + lane < paths) {
-#pragma unroll 1
-      for (int i = 0; i < kLsInputs; ++i) {
-        const float* rp = row_ptr(e, i);
-        if (rp) cp_async4(dst + i * T + lane, rp + qw + lane);
-      }
+#pragma unroll
+      for (int i = 0; i < kLsInputs; ++i)
+        if (src_s[e & 1][i]) cp_async4(dst + i * T + lane, src_s[e & 1][i] + qw + lane);
     }
     cp_async_commit();
   };
   auto start_date = [&](int e) {
-    if (R.vec16) {
-      rp0 = row_ptr(e, r0);
-      rp1 = row_ptr(e, r0 + 4);
-      rp2 = row_ptr(e, r0 + 8);
-    }
+    rp0 = src_s[e & 1][r0];
+    rp1 = src_s[e & 1][r0 + 4];
+    rp2 = src_s[e & 1][r0 + 8];
 #pragma unroll
     for (int k = 0; k < kLsStages - 1; ++k) issue(e, k, w0 + k * stride);
   };
@@ -803,6 +806,7 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
 #pragma unroll
     for (int i = 0; i < warp_sums_left<NP>(); ++i)
       if (i < count) red_s[warp][first + i] = (double)acc[i];
+    if (e > 0 && tid < kLsInputs) src_s[(e - 1) & 1][tid] = row_ptr(e - 1, tid);
     __syncthreads();
     double* part = ((E - 1 - e) & 1) ? part1 : part0;
     for (int q = tid; q < NP; q += T) {
@@ -876,8 +880,9 @@ __global__ void __launch_bounds__(LsThreads<KR>::value, 1)
     }
     return true;
   };
-  start_date(E - 1);
+  if (tid < kLsInputs) src_s[(E - 1) & 1][tid] = row_ptr(E - 1, tid);
   __syncthreads();
+  start_date(E - 1);
   for (int e = E - 1; e >= 0; --e) {
     bool ok;
     // the compile-time table where the date and the next (whose decision it
@@ -1128,7 +1133,7 @@ int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const 
                double* part, unsigned int* counter, double* gram, int* status,
                cudaStream_t s) {
   auto al16 = [](const void* q) { return ((uintptr_t)q & 15u) == 0; };
-  R.vec16 = (R.paths % 4 == 0) && al16(vars) && al16(cf) && al16(ex) && al16(num) && al16(y);
+  const bool vec16 = (R.paths % 4 == 0) && al16(vars) && al16(cf) && al16(ex) && al16(num) && al16(y);
   int slots = 0, votes[5] = {0, 0, 0, 0, 0}, kind = kBasisGeneric;
   for (int e = 0; e < R.n_ex; ++e) {
     slots = std::max(slots, R.date[e].nbasis + 1);
@@ -1154,8 +1159,10 @@ int launch_run(LSRun& R, int nblk, const float* vars, const float* means, const 
     return st ? st : check_launch("ls_run_kernel");
   };
 #define LMM_LS_RUN(KR, KIND)                                                            \
-  go(ls_run_kernel<KR, KIND>, KR*(KR + 1) / 2, ls_stage_bytes<KR, 1, false>(),          \
-     LsThreads<KR>::value)
+  (vec16 ? go(ls_run_kernel<KR, KIND, true>, KR*(KR + 1) / 2,                           \
+              ls_stage_bytes<KR, 1, false>(), LsThreads<KR>::value)                     \
+         : go(ls_run_kernel<KR, KIND, false>, KR*(KR + 1) / 2,                          \
+              ls_stage_bytes<KR, 1, false>(), LsThreads<KR>::value))
   switch (kind) {
     case kBasisC2: return LMM_LS_RUN(7, kBasisC2);
     case kBasisQuad: return LMM_LS_RUN(11, kBasisQuad);
