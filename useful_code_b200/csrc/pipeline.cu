@@ -578,12 +578,34 @@ int fused_price(const Validated& v, int P, const float* Z, const lmm_model* m,
   return fused_segments<kModeRule>(v, P, Z, m, rule, b, len, payoff, s);
 }
 
+// Level by level (variates_levels_kernel) where all CTAs of that form are
+// resident at once, at most five per SM, from 17 steps on.  Measured (depth
+// first, level by level): 40 steps, 5 factors 27, 20 us at 4,099 paths (165
+// CTAs), 24, 21 at 10,000 (395), alike at 20,481 (805); 80 steps, 10 factors 33,
+// 28 at 4,099 (330), 34, 35 at 10,000 (790); 120 steps, 15 factors 39, 28 at 1,000
+// (120), alike at 4,099 (495; 296 are resident), 20% for depth first at 6,000; 20
+// steps, 3 factors 10 to 30% for level by level up to 8,000 paths, 16 steps 9%
+// for depth first.
+bool variates_by_level(int n, int F, int P) {
+  if (n <= 16) return false;
+  const long long ctas = (long long)div_up(P, kVarBlock) * F;
+  const int per_sm = std::min<int>(5, 227 * 1024 / (int)(variates_levels_smem_bytes(n) + 1024));
+  return ctas <= (long long)per_sm * sm_count();
+}
+
 int launch_variates(const Validated& v, const lmm_model* m, int P, uint32_t off,
                     float* out, cudaStream_t s) {
   BridgePlan plan;
   TRY(make_bridge_plan(v.n, v.F, nullptr, &plan));
   LMM_REQUIRE((uint64_t)off + (uint64_t)P + 1u < (1ull << 31),
               "pipeline: Sobol point index must stay below 2^31");
+  if (variates_by_level(v.n, v.F, P)) {
+    const size_t smem = variates_levels_smem_bytes(v.n);
+    TRY(allow_smem((const void*)variates_levels_kernel, smem, "variates: smem attribute"));
+    variates_levels_kernel<<<dim3(div_up(P, kVarBlock), v.F), kVarBlock, smem, s>>>(
+        P, off + 1u, m->d_directions, m->d_scramblers, m->scramble_dims, out, plan);
+    return check_launch("variates_levels_kernel");
+  }
   VarPlan vp;
   make_var_plan(plan, &vp);
   const size_t smem = variates_smem_bytes(vp);
