@@ -273,3 +273,20 @@ def test_variates_by_level(cuda, n, F, P, offset):
     call("lmm_fused_variates", ctypes.addressof(pipe.model), size, offset - before, dp(many),
          stream_handle())
     assert torch.equal(few, many[:, :, before:before + P])
+
+
+@pytest.mark.parametrize("model,n,F", [("c3", 128, 10), ("c5", 120, 15), ("c2", 12, 2),
+                                       ("c2", 20, 3), ("c2", 14, 5), ("c3", 8, 10)])
+@pytest.mark.parametrize("product", ["swaption", "bermudan_cap"])
+def test_more_ctas_than_fit(cuda, model, n, F, product):
+    """One path per thread with more CTAs than the form that loads a step ahead
+    has places for (it reads rows and normals at the step then) against small
+    batches, which load ahead."""
+    pipe = pipeline(model, n, F, product=product)
+    P = 95001 if n * F <= 200 else 40001
+    whole, parts = pipe.first_pass(P, 777), pipe.first_pass(P, 777, batch=BATCH)
+    for name in ("vars", "ex", "cf", "num"):
+        assert torch.equal(getattr(whole, name), getattr(parts, name)), name
+    rule = pipe.regress(parts)
+    assert torch.equal(pipe.second_pass(P, 99999, rule),
+                       pipe.second_pass(P, 99999, rule, batch=BATCH))

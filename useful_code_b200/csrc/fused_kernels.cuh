@@ -562,9 +562,22 @@ __device__ __forceinline__ void stage_rows(float* As, float* fx, const float* __
 // displaced rate.  At exercise steps the discount ratios P(T_s, T_{r+1}),
 // the coterminal annuity and swap rate are accumulated on the fly.
 // FT = number of factors (compile time), 0 = generic <= 16.
+//
+// AHEAD costs registers and a second row buffer, so CTAs per SM.  Where not all
+// CTAs fit the SMs at once the other CTAs hide the loads, and the form without
+// it (rows and normals at the start of the step) holds more: 128 rates, 10
+// factors, 40,001 paths 1.85 against 1.40 ms (two against three CTAs per SM); 12
+// rates, 2 factors, 75,776 paths 61 against 50 us; 20 rates, 3 factors, the
+// European strip of 110,001 paths 87 against 70 us.
 // ---------------------------------------------------------------------------
-template <int FT, int MODE>
-__global__ void __launch_bounds__(kFusedBlock, FT > 0 && FT <= 5 ? 5 : 3)
+template <int FT, bool AHEAD>
+struct FusedShape {  // CTAs per SM that the registers have to allow
+  static constexpr int kCtas = AHEAD ? (FT == 3 || FT == 5 ? 5 : 3)
+                                     : FT == 3 ? 7 : FT == 5 ? 6 : 5;
+};
+
+template <int FT, int MODE, bool AHEAD>
+__global__ void __launch_bounds__(kFusedBlock, FusedShape<FT, AHEAD>::kCtas)
     fused_evolve_kernel(int paths, const float* __restrict__ Z,
                         const float* __restrict__ A,
                         const float* __restrict__ fixed,
@@ -589,11 +602,12 @@ __global__ void __launch_bounds__(kFusedBlock, FT > 0 && FT <= 5 ? 5 : 3)
   const int s_end = kSeg ? seg.s_end : n;
   const int rows = n - s_begin;  // rates alive in this launch
   extern __shared__ __align__(16) float sm[];
-  float* const As_b = sm;                     // [2][rows][FP]: row r - s of step s
-  float* const fx_b = As_b + 2 * rows * FP;   // [2][rows (+ pad)]
+  constexpr int kBufs = AHEAD ? 2 : 1;
+  float* const As_b = sm;                        // [kBufs][rows][FP]: row r - s of step s
+  float* const fx_b = As_b + kBufs * rows * FP;  // [kBufs][rows (+ pad)]
   const int fx_rows = (rows + 3) & ~3;
   // [rows][T], indexed by rate from s_begin on
-  float* const lfs = fx_b + 2 * fx_rows - s_begin * T;
+  float* const lfs = fx_b + kBufs * fx_rows - s_begin * T;
   int p = blockIdx.x * T + tid, src = 0;
   bool valid = p < paths;
   if (resume) {
@@ -620,12 +634,12 @@ __global__ void __launch_bounds__(kFusedBlock, FT > 0 && FT <= 5 ? 5 : 3)
       }
     }
   }
-  zero_row_pads<FP, T>(As_b, 2 * rows, F);
+  zero_row_pads<FP, T>(As_b, kBufs * rows, F);
   // copies step s's alive rows into buffer b
   auto stage = [&](int s, int b) {
     stage_rows<FT, FP, T>(As_b + b * rows * FP, fx_b + b * fx_rows, A, fixed, s, n, F);
   };
-  stage(s_begin, 0);
+  if (AHEAD) stage(s_begin, 0);
   float N = 1.0f, f_first = 0.0f, cf_acc = 0.0f, N_bucket = 1.0f;
   int bucket = -1, ex_at = n;
   double payoff = 0.0;
@@ -714,15 +728,20 @@ __global__ void __launch_bounds__(kFusedBlock, FT > 0 && FT <= 5 ? 5 : 3)
     for (int f = 0; f < FP; ++f)
       z_next[f] = (f < F && !done) ? __ldg(Z + ((size_t)s * F + f) * paths + p) : 0.0f;
   };
-  load_normals(s_begin);
+  if (AHEAD) load_normals(s_begin);
   for (int s = s_begin; s < s_end; ++s) {
+    if (!AHEAD) {
+      load_normals(s);
+      __syncthreads();  // every warp is past the step before's rows
+      stage(s, 0);
+    }
     cp_async_wait<0>();
     __syncthreads();  // this step's rows are in; the other buffer is free
-    const int buf = (s - s_begin) & 1;
+    const int buf = AHEAD ? (s - s_begin) & 1 : 0;
     float z[FP];
 #pragma unroll
     for (int f = 0; f < FP; ++f) z[f] = z_next[f];
-    if (s + 1 < s_end) {
+    if (AHEAD && s + 1 < s_end) {
       stage(s + 1, buf ^ 1);
       load_normals(s + 1);
     }
@@ -901,9 +920,9 @@ inline int launched_fm(int F) {
 inline int launched_row_pad(int F) { return (launched_fm(F) + 3) & ~3; }
 
 // Shared memory of the fused evolution kernel for `rows` alive rates.
-inline size_t fused_smem_bytes(int rows, int F, int block) {
+inline size_t fused_smem_bytes(int rows, int F, bool ahead) {
   const size_t stage = (size_t)rows * launched_row_pad(F) + ((rows + 3) & ~3);
-  return (2 * stage + (size_t)rows * block) * sizeof(float);
+  return ((ahead ? 2 : 1) * stage + (size_t)rows * kFusedBlock) * sizeof(float);
 }
 // The same with one buffer (greeks_segment_kernel).
 inline size_t segment_smem_bytes(int rows, int F, int block) {

@@ -438,6 +438,18 @@ int evolve_block(const Validated& v, int P, bool chain) {
   return use_pairs(v, P, chain) ? kPairBlock : kFusedBlock;
 }
 
+// fused_evolve_kernel with its loads a step ahead: where all CTAs of that form
+// are resident at once (its registers allow 5, 4 or 3 per SM by factors), and in
+// chains of 3 or 5 factors, whose CTAs empty as paths exercise (40 rates, 5
+// factors 1.10, 64 rates, 3 factors 1.03 times as fast so at 95,000 paths).
+bool fused_ahead(int rows, int F, int grid, bool chain) {
+  const bool few = F == 3 || F == 5;
+  if (chain && few) return true;
+  const int regs = few ? 5 : F == 10 ? 4 : 3;
+  const int smem = (int)(228 * 1024 / (fused_smem_bytes(rows, F, true) + 1024));
+  return grid <= std::min(regs, smem) * sm_count();
+}
+
 template <int MODE>
 int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
                  const LsRuleView& rule,
@@ -454,8 +466,10 @@ int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
   const SegIO& sg = segment ? *segment : whole;
   const int rows = v.n - sg.s_begin;  // rates alive at the launch's first step
   const int tmem_rows = pairs ? pair_tmem_rows(rows, v.F) : 0;
+  constexpr bool kLight = MODE == kModeInputs || MODE == kModeRule;
+  const bool ahead = !kLight || fused_ahead(rows, v.F, grid, segment != nullptr);
   const size_t smem = pairs ? pair_smem_bytes(rows, v.F, rows - tmem_rows)
-                                   : fused_smem_bytes(rows, v.F, block);
+                            : fused_smem_bytes(rows, v.F, ahead);
   auto attr = [&](auto kern) -> int {
     return allow_smem((const void*)kern, smem, "fused: smem attribute");
   };
@@ -468,11 +482,15 @@ int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
           payoff, rec, sg, v.n - tmem_rows);
       return check_launch("fused_pairs_kernel");
     }
-    TRY(attr(fused_evolve_kernel<FT, MODE>));
-    fused_evolve_kernel<FT, MODE><<<grid, block, smem, s>>>(
-        P, Z, m->d_A, m->d_fixed_drifts, v.mc, v.pc, v.rc, rule, total, col, vars, ex, cf, num,
-        payoff, rec, sg);
-    return check_launch("fused_evolve_kernel");
+    auto one = [&](auto kern) -> int {
+      TRY(attr(kern));
+      kern<<<grid, block, smem, s>>>(P, Z, m->d_A, m->d_fixed_drifts, v.mc, v.pc, v.rc, rule,
+                                     total, col, vars, ex, cf, num, payoff, rec, sg);
+      return check_launch("fused_evolve_kernel");
+    };
+    if constexpr (kLight)
+      if (!ahead) return one(fused_evolve_kernel<FT, MODE, false>);
+    return one(fused_evolve_kernel<FT, MODE, true>);
   });
 }
 
