@@ -204,7 +204,7 @@ def test_threads_price_at_once(cuda):
 
 
 # the reverse sweep takes two paths per thread from 75,777 paths (593 tiles, up
-# to 10 factors) and the recompute from 56,000 (n F P >= 2^23); 15 factors and
+# to 10 factors) and the recompute from 56,833 (n F P >= 2^23); 15 factors and
 # the generic form keep one in the reverse sweep
 @pytest.mark.parametrize("model,n,F,P,product", [
     ("c3", 80, 10, 100004, "swaption"), ("c2", 40, 5, 81932, "cancellable"),
@@ -236,8 +236,8 @@ def test_greeks_batches(cuda, model, n, F, P, product):
         assert np.linalg.norm(got - ref) < 3.8e-6 * np.linalg.norm(ref), name
 
 
-@pytest.mark.parametrize("model,n,F,K", [("c3", 16, 10, 56007), ("c2", 30, 5, 56004),
-                                         ("c3", 50, 3, 56001), ("c5", 28, 15, 20485),
+@pytest.mark.parametrize("model,n,F,K", [("c3", 16, 10, 57007), ("c2", 30, 5, 57004),
+                                         ("c3", 50, 3, 57001), ("c5", 28, 15, 20485),
                                          ("c3", 27, 16, 20483)])
 def test_bound_outer_paths(cuda, model, n, F, K):
     """Outer paths of the Andersen-Broadie bound, two per thread, against a
@@ -275,8 +275,21 @@ def test_variates_by_level(cuda, n, F, P, offset):
     assert torch.equal(few, many[:, :, before:before + P])
 
 
+# chains of segments take two paths per thread later than one launch does
+@pytest.mark.parametrize("model,n,F,P", [("c3", 80, 10, 110011), ("c2", 40, 5, 250017),
+                                         ("c5", 120, 15, 150011), ("c2", 64, 3, 262147),
+                                         ("c3", 128, 10, 100481)])
+@pytest.mark.parametrize("product", ["swaption", "cancellable"])
+def test_chain_batches(cuda, model, n, F, P, product):
+    """A chain with two paths per thread against batches with one."""
+    pipe = pipeline(model, n, F, product=product)
+    rule = pipe.regress(pipe.first_pass(8192, 0))
+    whole = pipe.second_pass(P, 99999, rule)
+    assert torch.equal(whole, pipe.second_pass(P, 99999, rule, batch=BATCH))
+
+
 @pytest.mark.parametrize("model,n,F", [("c3", 128, 10), ("c5", 120, 15), ("c2", 12, 2),
-                                       ("c2", 20, 3), ("c2", 14, 5), ("c3", 8, 10)])
+                                       ("c2", 20, 3), ("c2", 14, 5), ("c3", 20, 10)])
 @pytest.mark.parametrize("product", ["swaption", "bermudan_cap"])
 def test_more_ctas_than_fit(cuda, model, n, F, product):
     """One path per thread with more CTAs than the form that loads a step ahead

@@ -418,24 +418,54 @@ int dispatch_factors(int F, Fn&& go) {
   }
 }
 
-// Two paths per thread (fused_pairs.cuh) where the pairs still fill the GPU,
-// else one: with fewer paths the halved number of warps costs more than the
-// pairs save.  Measured (one against two paths per thread): one launch of 80
-// rates and 10 factors 0.60 / 0.67 ms at 50,000 paths, 0.76 / 0.67 at 65,536,
-// 1.44 / 1.22 at 150,000; of 120 rates and 15 factors 1.20 / 1.11 at 20,480,
-// 2.37 / 1.80 at 65,536; of 40 rates and 5 factors 0.129 / 0.145 at 37,000,
-// 0.181 / 0.175 at 65,536, 0.55 / 0.44 at 2^18.  In a chain of segments the
-// later launches hold few survivors: 80 rates 0.87 / 0.95 at 65,536, 1.21 /
-// 1.15 at 110,000; 120 rates 1.83 / 2.05 at 65,536; 40 rates 0.32 / 0.35 at
-// 110,000.  Few rates and factors (20 and 3: 57 / 62 us at 65,536) leave a
-// step too little arithmetic to pair.
-bool use_pairs(const Validated& v, int P, bool chain) {
-  if ((long long)P * v.n * v.F < (1ll << 23)) return false;
-  if (chain) return P >= (v.F >= 10 ? 100000 : 160000);
-  return P >= (v.F > 10 ? 20480 : 56000);
+// Two paths per thread (fused_pairs.cuh) where that beats one per thread: the
+// pairs halve the warps, so with few paths they leave the SMs short of them.
+// `mode` is the launch's (-1: the Greeks' recompute).  Measured, one against two
+// paths per thread in ms at the paths beside it:
+//   One launch that writes the LS inputs: 80 rates, 10 factors 0.59 / 0.66 at
+// 56,001 (the last that keep three one-path CTAs per SM), 0.75 / 0.67 at 57,000,
+// 1.26 / 1.21 at 130,000; 40 rates, 5 factors 0.151 / 0.175, 0.181 / 0.174,
+// 0.30 / 0.27; 30 rates, 16 factors 0.150 / 0.171, 0.190 / 0.170, 0.30 / 0.30.
+// 120 rates, 15 factors also between one and two one-path CTAs per SM, 1.20 / 1.11
+// at 20,481 (1.66 / 1.79 at 40,001; 30 rates, 16 factors 0.113 / 0.122 at 20,481).
+//   One launch with the frozen rule or without exercise: as above from 2^24
+// rates x factors x paths on (40 rates, 5 factors 0.215 / 0.243 at 57,000, 0.36 /
+// 0.29 at 95,000; 20 rates, 3 factors, the European strip 0.101 / 0.110 at
+// 160,001, 0.175 / 0.142 at 300,001).  The generic factor count gains little per
+// path (60 rates, 8 factors 3.2 / 3.1 at 400,001): up to four one-path CTAs per SM
+// (the European strip 0.59 / 0.54 at 65,536, the frozen rule 0.69 / 0.70), and
+// beyond only where it saves a wave of CTAs: 0.98 / 0.91 at 95,000 (five one-path
+// CTAs per SM, 94,720 paths, against three pair CTAs, 113,664), but 1.12 / 1.26 at
+// 130,000.
+//   Chains of segments, whose later launches hold few survivors: 80 rates, 10
+// factors 1.11 / 1.11 at 95,000, 1.20 / 1.15 at 110,001; 40 rates, 10 factors
+// 0.59 / 0.61 at 200,000, 0.77 / 0.73 at 2^18; 120 rates, 15 factors 2.37 / 2.48
+// at 110,001, 2.75 / 2.76 at 130,000, 3.2 / 3.1 at 160,001; 40 rates, 5 factors
+// 0.48 / 0.49 at 200,001, 0.62 / 0.61 at 300,001; the generic count never (30
+// rates, 16 factors 0.46 / 0.54 at 200,001, 0.82 / 0.88 at 400,001).
+bool use_pairs(const Validated& v, int P, bool chain, int mode) {
+  const bool few = v.F == 3 || v.F == 5, compiled = few || v.F == 10 || v.F == 15;
+  const long long work = (long long)P * v.n * v.F;
+  if (chain) {
+    if (!compiled) return false;
+    if (few) return P >= 160000 && work >= 50000000;
+    return P >= (v.F > 10 ? 150000 : 100000) && work >= 88000000;
+  }
+  const int sms = sm_count();
+  if (mode == kModeRule) {
+    if (work < (1ll << 24) || P <= 3 * kFusedBlock * sms) return false;
+    // a pair wave lasts about as long as its paths' share of one-path waves
+    const int one_wave = 5 * kFusedBlock * sms, pair_wave = 3 * kPairBlock * sms;
+    return compiled || P <= 4 * kFusedBlock * sms ||
+           (long long)div_up(P, pair_wave) * pair_wave < (long long)div_up(P, one_wave) * one_wave;
+  }
+  if (work < (1ll << 23)) return false;
+  if (P > 3 * kFusedBlock * sms) return true;
+  if (v.F <= 10 || P < 20480) return false;
+  return mode != kModeInputs || (v.n >= 100 && P <= 2 * kFusedBlock * sms);
 }
 int evolve_block(const Validated& v, int P, bool chain) {
-  return use_pairs(v, P, chain) ? kPairBlock : kFusedBlock;
+  return use_pairs(v, P, chain, kModeRule) ? kPairBlock : kFusedBlock;
 }
 
 // fused_evolve_kernel with its loads a step ahead: where all CTAs of that form
@@ -457,7 +487,7 @@ int launch_fused(const Validated& v, int P, const float* Z, const lmm_model* m,
                  float* num, float* payoff, cudaStream_t s,
                  RecordOut rec = RecordOut{nullptr, nullptr, nullptr, 1},
                  const SegIO* segment = nullptr) {
-  const bool pairs = use_pairs(v, P, segment != nullptr);
+  const bool pairs = use_pairs(v, P, segment != nullptr, MODE);
   const int block = pairs ? kPairBlock : kFusedBlock;
   const int grid = div_up(P, block);
   SegIO whole{};
@@ -578,7 +608,13 @@ int fused_segments(const Validated& v, int P, const float* Z, const lmm_model* m
 // 65,536, 1.12, 1.08, 1.09 at 95,000; 120 rates, 15 factors 1.25, 1.15, 1.01 at
 // 18,944, 1.33, 1.22, 1.45 at 30,000, 1.83, 1.80, 2.06 at 65,536, 2.33, 2.39,
 // 2.83 at 95,000; 40 rates, 5 factors 0.21, 0.18, 0.16 at 18,944, 0.26, 0.23,
-// 0.25 at 65,536.
+// 0.25 at 65,536.  The line goes by CTAs per SM alone and is not the best for
+// every model: between one and three CTAs per SM one launch is up to 10% faster
+// than 16 steps at 80 rates, 10 factors (0.59, 0.53 ms at 30,000 paths) and 40
+// rates, 5 factors (0.18, 0.16), and as much slower at 120 rates, 15 factors (1.21,
+// 1.30); segments of 27 steps are 2 to 6% faster than 16 up to four CTAs per SM
+// (0.56 at 30,000, 0.77 against 0.81 at 65,536; 1.21 and 1.95 against 1.22 and
+// 1.80 at 120 rates).
 int default_segment(const Validated& v, int P) {
   const int ctas = div_up(P, kFusedBlock);
   return ctas <= sm_count() ? v.n : ctas <= 4 * sm_count() ? 2 * kSegSteps : kSegSteps;
@@ -1117,7 +1153,7 @@ extern "C" int lmm_greeks(const lmm_model* model, const lmm_product* product,
   const double P0 = 1.0 / (1.0 + (double)model->h_initial_rates[0] * (double)t0);
   const double scale = P0 / (double)P;
   // the recompute: one tile of the reverse sweep per CTA, or two with pairs
-  const bool pairs = use_pairs(v, P, false);
+  const bool pairs = use_pairs(v, P, false, -1);
   const int block_seg = pairs ? kPairBlock : kRevThreads;
   auto seg_smem = [&](int s0) {
     return pairs ? pair_smem_bytes(n - s0, F, n - s0 - pair_tmem_rows(n - s0, F))
