@@ -701,9 +701,13 @@ size_t greeks_seg_floats(size_t n, size_t P, int k) {
 }
 
 // Upper bound on the CTAs of the reverse kernel (sizes the partials, and bounds
-// the launch): its register counts, 110 to 224, let an SM hold four at most.
+// the launch): its register counts, 110 to 224, let an SM hold four at most.  At
+// least 32, although fewer tiles leave CTAs without paths: each launch's warps
+// also sum the launch before's partials, 8 n (F + 1) entries, which one CTA took
+// 1.2 ms for (80 rates, 10 factors, 4 paths: 12.5 -> 2.6 ms a call).  Their
+// partials are zeros, so the sums are the same.
 int greeks_reverse_grid(int P) {
-  return std::min(div_up(P, kRevThreads), 4 * sm_count());
+  return std::min(std::max(div_up(P, kRevThreads), 32), 4 * sm_count());
 }
 
 GreeksBufs carve_greeks(Carver& c, const Validated& v, size_t P, int k) {
