@@ -598,11 +598,13 @@ def run_b200(args) -> int:
     traffic = None
     tf = ROOT / "profiles" / "traffic.json"
     if tf.exists():
-        per_path = json.loads(tf.read_text()).get(f"fused_evolve_{args.config}_bytes_per_path")
-        if per_path is not None and t_first is not None:
+        per_path = json.loads(tf.read_text()).get(f"first_pass_{args.config}_bytes_per_path")
+        if per_path is not None and t_first is not None and not tensor:
             traffic = per_path * Preg
-    kname = "tc_evolve_kernel" if tensor else "fused_pairs_kernel"
-    roofline = {"bound": "fp32", "kernel": f"{kname} (first pass)",
+    # the fused form runs as one or two paths per thread by paths, rates and factors
+    kname = "tc_evolve_kernel" if tensor else "fused evolution"
+    which = "first pass" if t_first is not None else "second pass"
+    roofline = {"bound": "fp32", "kernel": f"{kname} ({which})",
                 "achieved": achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                 "frac": achieved / fp32_peak, "traffic": traffic,
                 "peak_source": "nominal FP32 FMA rate, 148 SMs x 128 lanes x 2 at the median "
