@@ -415,8 +415,10 @@ int lmm_step_to_exercise_indices(const int* h_gen_indices, int n_gen,
  * With at most 10 functions per date the backward loop is one cooperative
  * launch of at most one CTA per SM; on a stream that owns too few SMs for it
  * (a green context's), and with more functions, it is one launch per date,
- * with the same results to the last bit.  Two regressions on two streams may
- * therefore run one after the other.  The call can be captured in a graph. */
+ * with the same results to the last bit.  Regressions on two streams overlap
+ * while their CTAs (one per 512 paths, at most one per SM) fit the GPU
+ * together, and run one after the other beyond.  The call can be captured in a
+ * graph. */
 size_t lmm_ls_workspace_bytes(int paths, int n_exercise);
 int lmm_ls_regress(int n_exercise, int paths, const float* d_vars,
                    const int* h_nvars, const uint8_t* h_monomials,

@@ -204,10 +204,13 @@ def test_threads_price_at_once(cuda):
 
 
 # the reverse sweep takes two paths per thread from 75,777 paths (593 tiles, up
-# to 10 factors) and the recompute from 56,833 (n F P >= 2^23); 15 factors and
-# the generic form keep one in the reverse sweep
+# to 10 factors), the recompute and a recording pass in one launch from 56,833
+# (n F P >= 2^23), a recording pass in segments as test_chain_batches; 15 factors
+# and the generic form keep one in the reverse sweep
 @pytest.mark.parametrize("model,n,F,P,product", [
-    ("c3", 80, 10, 100004, "swaption"), ("c2", 40, 5, 81932, "cancellable"),
+    ("c3", 80, 10, 110004, "swaption"), ("c2", 40, 5, 81932, "cancellable"),
+    ("c2", 40, 5, 250020, "swaption"), ("c5", 120, 15, 150004, "cancellable"),
+    ("c2", 64, 3, 262148, "swaption"),
     ("c3", 24, 10, 77828, "bermudan_cap"), ("c1", 28, 5, 75780, "european"),
     ("c2", 37, 3, 82052, "swaption"), ("c5", 30, 15, 60004, "swaption"),
     ("c3", 21, 16, 57004, "cancellable")])
