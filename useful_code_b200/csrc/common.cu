@@ -95,7 +95,11 @@ int stream_sm_count(cudaStream_t s) {
 int allow_smem(const void* kern, size_t bytes, const char* what) {
   cudaFuncAttributes fa;
   int st = check_cuda(cudaFuncGetAttributes(&fa, kern), what);
-  if (st || bytes <= (size_t)fa.maxDynamicSharedSizeBytes) return st;
+  if (st) return st;
+  constexpr size_t kUnasked = 48 * 1024;  // static and dynamic, without asking
+  const size_t limit = (size_t)fa.maxDynamicSharedSizeBytes;
+  if (bytes + fa.sharedSizeBytes <= kUnasked || (limit > kUnasked && bytes <= limit))
+    return LMM_OK;
   int dev = 0, most = 0;
   st = check_cuda(cudaGetDevice(&dev), what);
   if (st) return st;
