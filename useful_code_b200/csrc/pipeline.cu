@@ -701,13 +701,16 @@ size_t greeks_seg_floats(size_t n, size_t P, int k) {
 }
 
 // Upper bound on the CTAs of the reverse kernel (sizes the partials, and bounds
-// the launch): its register counts, 110 to 224, let an SM hold four at most.  At
-// least 32, although fewer tiles leave CTAs without paths: each launch's warps
-// also sum the launch before's partials, 8 n (F + 1) entries, which one CTA took
-// 1.2 ms for (80 rates, 10 factors, 4 paths: 12.5 -> 2.6 ms a call).  Their
-// partials are zeros, so the sums are the same.
+// the launch): its register counts, 110 to 224, let an SM hold four at most.  One
+// per tile of every chunk, those that the last chunk lacks included: a CTA
+// without paths adds zeros, but with fewer CTAs than places in the chunks one
+// CTA had two tiles while others had none, and every step took twice as long (120
+// rates, 15 factors, the swaption-plus-cap portfolio of 12,000 paths 10.2 -> 7.0
+// ms a call); and each launch's warps also sum the launch before's partials, 8 n
+// (F + 1) entries, which one CTA took 1.2 ms for (80 rates, 10 factors, 4 paths
+// 12.5 -> 2.6 ms).
 int greeks_reverse_grid(int P) {
-  return std::min(std::max(div_up(P, kRevThreads), 32), 4 * sm_count());
+  return std::min(div_up(P, kSortChunk) * (kSortChunk / kRevThreads), 4 * sm_count());
 }
 
 GreeksBufs carve_greeks(Carver& c, const Validated& v, size_t P, int k) {
