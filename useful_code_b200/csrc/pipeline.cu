@@ -430,13 +430,17 @@ int dispatch_factors(int F, Fn&& go) {
 // at 20,481 (1.66 / 1.79 at 40,001; 30 rates, 16 factors 0.113 / 0.122 at 20,481).
 //   One launch with the frozen rule or without exercise: as above from 2^24
 // rates x factors x paths on (40 rates, 5 factors 0.215 / 0.243 at 57,000, 0.36 /
-// 0.29 at 95,000; 20 rates, 3 factors, the European strip 0.101 / 0.110 at
-// 160,001, 0.175 / 0.142 at 300,001).  The generic factor count gains little per
-// path (60 rates, 8 factors 3.2 / 3.1 at 400,001): up to four one-path CTAs per SM
-// (the European strip 0.59 / 0.54 at 65,536, the frozen rule 0.69 / 0.70), and
-// beyond only where it saves a wave of CTAs: 0.98 / 0.91 at 95,000 (five one-path
-// CTAs per SM, 94,720 paths, against three pair CTAs, 113,664), but 1.12 / 1.26 at
-// 130,000.
+// 0.29 at 95,000), below where the pairs save a wave of CTAs (20 rates, 3 factors,
+// the European strip 0.101 / 0.110 at 160,001, 0.129 / 0.110 at 140,001: one wave of
+// 151,552 paths against two of 132,608).  The generic factor count gains little per
+// path (60 rates, 8 factors 3.2 / 3.1 at 400,001): for the European strip (0.59 /
+// 0.54 at 65,536, 1.48 / 1.38 at 200,001), up to four one-path CTAs per SM (the
+// frozen rule 0.69 / 0.70 at 65,536), and beyond only where it saves a wave: 0.98 /
+// 0.91 at 95,000, but 1.12 / 1.26 at 130,000.
+//   The swaption-plus-cap portfolio's, whose paths run to the last step, from one
+// one-path CTA per SM on: 80 rates, 10 factors 0.89 / 0.66 at 20,481, 1.13 / 0.85 at
+// 56,001; 120 rates, 15 factors 2.3 / 1.5 at 20,481; 30 rates, 16 factors 0.18 / 0.22
+// at 18,944, 0.21 / 0.22 at 20,481, 0.26 / 0.23 at 37,889.
 //   Chains of segments, whose later launches hold few survivors: 80 rates, 10
 // factors 1.11 / 1.11 at 95,000, 1.20 / 1.15 at 110,001; 40 rates, 10 factors
 // 0.59 / 0.61 at 200,000, 0.77 / 0.73 at 2^18; 120 rates, 15 factors 2.37 / 2.48
@@ -452,14 +456,19 @@ bool use_pairs(const Validated& v, int P, bool chain, int mode) {
     return P >= (v.F > 10 ? 150000 : 100000) && work >= 88000000;
   }
   const int sms = sm_count();
-  if (mode == kModeRule) {
-    if (work < (1ll << 24) || P <= 3 * kFusedBlock * sms) return false;
-    // a pair wave lasts about as long as its paths' share of one-path waves
-    const int one_wave = 5 * kFusedBlock * sms, pair_wave = 3 * kPairBlock * sms;
-    return compiled || P <= 4 * kFusedBlock * sms ||
-           (long long)div_up(P, pair_wave) * pair_wave < (long long)div_up(P, one_wave) * one_wave;
-  }
   if (work < (1ll << 23)) return false;
+  if (v.pc.kind == LMM_PRODUCT_BERMUDAN_CAP && (mode == kModeRule || mode == kModeRecord))
+    return P > kFusedBlock * sms;
+  if (mode == kModeRule) {
+    if (P <= 3 * kFusedBlock * sms) return false;
+    const bool enough = work >= (1ll << 24) &&
+                        (compiled || v.pc.kind == LMM_PRODUCT_EUROPEAN ||
+                         P <= 4 * kFusedBlock * sms);
+    // otherwise where it saves a wave of CTAs: a wave lasts about as its paths
+    const long long one_wave = (few ? v.F == 3 ? 7 : 6 : 5) * kFusedBlock * sms,
+                    pair_wave = (few ? 4 : 3) * kPairBlock * sms;
+    return enough || div_up(P, pair_wave) * pair_wave < div_up(P, one_wave) * one_wave;
+  }
   if (P > 3 * kFusedBlock * sms) return true;
   if (v.F <= 10 || P < 20480) return false;
   return mode != kModeInputs || (v.n >= 100 && P <= 2 * kFusedBlock * sms);
