@@ -94,9 +94,9 @@ def test_variates_pieces(cuda, n, F, P, offset):
 
 @pytest.mark.parametrize("n", [2, 3, 4, 5, 7, 8, 9, 16, 31, 33, 63, 64, 65, 100, 127, 128])
 def test_variates_depth_first_bridge(cuda, n):
-    """Every tree shape of the depth-first bridge (above 16 steps, where 300
-    paths run level by level: the first of 60,000, three tiles or more per SM)
-    against the level-by-level construction in FP64 on exact normals.  Bridge values reach 6 sqrt(128) =
+    """Every tree shape of the depth-first bridge (the first of 100,000 paths) and
+    of the level-by-level one (300 paths alone) against the construction in FP64
+    on exact normals.  Bridge values reach 6 sqrt(128) =
     68; an FP32 combination rounds them by up to 68 * 2^-23 = 8e-6 per level
     (at most eight levels) and the rational inverse normal is within 7e-7
     relative of the exact one: 1e-4 bounds the difference of two points."""
@@ -122,10 +122,9 @@ def test_variates_depth_first_bridge(cuda, n):
                  model.d_A, model.d_fixed_drifts, dp(d_dirs), dp(d_scr), F * n_, 10.0)
     out = torch.empty(n_, F, P, device="cuda")
     call("lmm_fused_variates", ctypes.addressof(m), P, offset, dp(out), stream_handle())
-    if n > 16:
-        many = torch.empty(n_, F, 60000, device="cuda")
-        call("lmm_fused_variates", ctypes.addressof(m), 60000, offset, dp(many), stream_handle())
-        assert torch.equal(many[:, :, :P], out)
+    many = torch.empty(n_, F, 100000, device="cuda")
+    call("lmm_fused_variates", ctypes.addressof(m), 100000, offset, dp(many), stream_handle())
+    assert torch.equal(many[:, :, :P], out)
     lw, rw, sd = (np.zeros(n_) for _ in range(3))
     left, right, bidx = (np.zeros(n_, np.int32) for _ in range(3))
     call("lmm_bridge_tables_host", n_, *(vp(a.ctypes.data)
@@ -259,11 +258,13 @@ def test_bound_outer_paths(cuda, model, n, F, K):
         assert torch.equal(getattr(whole, name)[..., K - 257:], getattr(tail, name)), name
 
 
-@pytest.mark.parametrize("n,F", [(17, 3), (20, 3), (40, 5), (80, 10), (128, 16)])
+@pytest.mark.parametrize("n,F", [(2, 1), (2, 2), (16, 4), (20, 3), (40, 5), (80, 10),
+                                 (128, 16)])
 @pytest.mark.parametrize("P,offset", [(1, 0), (127, 126), (129, 127), (4099, 2**31 - 4102)])
 def test_variates_by_level(cuda, n, F, P, offset):
     """Few paths (level by level, tiles of 128) against the same paths inside a
-    launch with many (depth first); the last offset ends at the last index."""
+    launch with many (depth first; one factor stays level by level up to 94,720
+    paths); the last offset ends at the last index."""
     from useful_code_b200._lib import call
     from useful_code_b200.pricer import dp, stream_handle
 

@@ -385,9 +385,9 @@ inline size_t variates_smem_bytes(const VarPlan& p) {
 // CTAs leave the SMs nearly empty, which last as long as one thread's chain.
 // Depth first every point waits for the point before it, and the increments
 // come out in between; level by level the points of a level are independent.
-// Per launch, depth first and so: 80 steps, 10 factors 30 -> 22 us at 1,000
-// paths, 33 -> 28 at 4,099; 128 steps, 16 factors 41 -> 27 us at 1,000; 40
-// steps, 5 factors 27 -> 20 us at 4,099, 24 -> 21 at 10,000.
+// On the device, depth first and so: 80 steps, 10 factors 16.7 -> 8.7 us at
+// 1,000 paths, 18.7 -> 13.8 at 4,099; 128 steps, 16 factors 24.2 -> 12.5 us at
+// 1,000; 40 steps, 5 factors 9.7 -> 7.0 us at 4,099.
 __global__ void __launch_bounds__(kVarBlock)
     variates_levels_kernel(int paths, uint32_t first_index, const uint32_t* __restrict__ dirs,
                            const uint32_t* __restrict__ scr, int scr_dims,

@@ -642,15 +642,14 @@ int fused_price(const Validated& v, int P, const float* Z, const lmm_model* m,
 }
 
 // Level by level (variates_levels_kernel) where all CTAs of that form are
-// resident at once, at most five per SM, from 17 steps on.  Measured (depth
-// first, level by level): 40 steps, 5 factors 27, 20 us at 4,099 paths (165
-// CTAs), 24, 21 at 10,000 (395), alike at 20,481 (805); 80 steps, 10 factors 33,
-// 28 at 4,099 (330), 34, 35 at 10,000 (790); 120 steps, 15 factors 39, 28 at 1,000
-// (120), alike at 4,099 (495; 296 are resident), 20% for depth first at 6,000; 20
-// steps, 3 factors 10 to 30% for level by level up to 8,000 paths, 16 steps 9%
-// for depth first.
+// resident at once, at most five per SM.  Measured on the device (depth first,
+// level by level, us): 8 steps, 4 factors 3.7, 3.2 at 4,099 paths (132 CTAs), 4.3,
+// 4.2 at 20,481 (644), 5.1, 5.5 at 40,001 (1,252); 16 steps, 16 factors 5.1, 3.9 at
+// 1,000 (128), 7.0, 7.4 at 8,000 (1,008); 40 steps, 5 factors 9.7, 7.0 at 4,099
+// (165), 12.3, 12.8 at 20,481 (805); 80 steps, 10 factors 16.7, 8.7 at 1,000 (80),
+// 21.7, 20.8 at 8,000 (630; 592 are resident), 25.5, 29.2 at 14,000; 120 steps, 15
+// factors 23.0, 11.7 at 1,000 (120), 26.8, 29.6 at 4,099 (495; 296 are resident).
 bool variates_by_level(int n, int F, int P) {
-  if (n <= 16) return false;
   const long long ctas = (long long)div_up(P, kVarBlock) * F;
   const int per_sm = std::min<int>(5, 227 * 1024 / (int)(variates_levels_smem_bytes(n) + 1024));
   return ctas <= (long long)per_sm * sm_count();
