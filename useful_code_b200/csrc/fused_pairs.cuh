@@ -29,14 +29,16 @@ struct PairShape {
 // (256 KB per SM that this kernel has no other use for): rates nt0 .. n - 1
 // as columns of the CTA's allocation, lane = thread, read and written four
 // rates (eight columns) at a time; the rates below nt0 in shared memory.
-// That makes room for four CTAs (1,024 paths) per SM at 80 rates and 10
-// factors, as many as the registers allow.
+// That makes room for as many CTAs per SM as the registers allow, three (768
+// paths) at 80 rates and 10 factors; fewer than 53 rates of 3 or 5 factors, or
+// 67 of more, fit shared memory whole (pair_tmem_rows).
 //
 // One path per thread with all log-rates in shared memory, two paths per
 // thread with them there, and this form: 80 rates, 10 factors, 2^20 paths 9.79,
 // 8.83, 7.69 ms (FMA pipe 50, 57, 65% busy), its frozen-rule chain 8.93, 7.68
 // (with the known basis tables), 7.1; 120 rates, 15 factors, 2^18 paths 8.07,
-// 7.40, 5.70; 40 rates, 5 factors, 2^18 paths 0.61, 0.47, 0.44.  A software-
+// 7.40, 5.70; 40 rates, 5 factors, 2^18 paths (all in shared memory; 128 threads
+// per CTA and the row copies make the last difference) 0.61, 0.47, 0.44.  A software-
 // pipelined rate loop (three consecutive blocks of rates in three stages) was
 // slower: 9.55 ms with 26% more instructions.  At 10 factors three CTAs of 168
 // registers beat four of 128 (7.69 against 7.83 ms).
