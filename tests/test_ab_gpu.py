@@ -166,7 +166,7 @@ def test_bounds_bracket_the_price(swaption_rules):
                                          ("c3", 75, 16, 5), ("c2", 59, 3, 1)])
 def test_inner_estimates_of_large_models(cuda, model, n, F, K):
     """Every compiled factor count and the generic one, at rate counts whose
-    last log-rates lie in tensor memory (from 53 rates of 3 or 5 factors and 67
+    last log-rates lie in tensor memory (from 54 rates of 3 or 5 factors and 69
     of more), with an odd number of 128-path units per date, so that
     one warp pair of the last CTA is idle: continuation estimates against the
     oracle on the device's outer states and the same normals.  A flipped inner

@@ -30,8 +30,8 @@ struct PairShape {
 // as columns of the CTA's allocation, lane = thread, read and written four
 // rates (eight columns) at a time; the rates below nt0 in shared memory.
 // That makes room for as many CTAs per SM as the registers allow, three (768
-// paths) at 80 rates and 10 factors; fewer than 53 rates of 3 or 5 factors, or
-// 67 of more, fit shared memory whole (pair_tmem_rows).
+// paths) at 80 rates and 10 factors; up to 52 rates of 3 or 5 factors, or 66
+// of more, fit shared memory whole (pair_tmem_rows).
 //
 // One path per thread with all log-rates in shared memory, two paths per
 // thread with them there, and this form: 80 rates, 10 factors, 2^20 paths 9.79,
